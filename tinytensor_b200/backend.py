@@ -80,6 +80,7 @@ def _shape_str(t) -> str:
     return "(" + ", ".join(str(int(d)) for d in t.shape) + ")"
 
 _lib = None
+_fast = None  # csrc/torch_ext.cpp: the native call path of the functions below
 
 
 def lib_path() -> Path:
@@ -163,9 +164,34 @@ def lib() -> ctypes.CDLL:
     return L
 
 
+def _native():
+    """The extension module that calls the C ABI straight from torch tensors (csrc/torch_ext.cpp).
+    Its functions return None for calls that are not the ordinary case; the Python code that
+    follows each use then converts, checks and names the error."""
+    global _fast
+    L = lib()
+    if _fast is None:
+        try:
+            from . import _ttb_torch
+        except ImportError as e:
+            raise TTBError(f"the call-path extension is not built ({e}): build it with `python -m tinytensor_b200.build`") from e
+        names = ("ttb_batched_matmul", "ttb_batched_matmul_strided_out", "ttb_batched_matmul_fused", "ttb_conv2d_forward",
+                 "ttb_conv2d_backward")
+        _ttb_torch.bind(*(ctypes.cast(getattr(L, n), ctypes.c_void_p).value for n in names))
+        _fast = _ttb_torch
+    return _fast
+
+
 def _raise(status: int) -> None:
     msg = lib().ttb_last_error().decode("utf-8", "replace")
     raise TTBError(msg or f"ttb status {status}", status)
+
+
+def _checked(r):
+    """A result of the native call path: what it computed, or a status to raise."""
+    if r.__class__ is int:
+        _raise(r)
+    return r
 
 
 def _make_view(data_ptr: int, offset: int, sizes, strides) -> _View:
@@ -242,6 +268,9 @@ def batched_matmul(lhs: torch.Tensor, rhs: torch.Tensor, out: torch.Tensor | Non
     `out` (rank 3, any strides) is given.  Queued on the current torch stream; does not
     synchronise.
     """
+    r = (_fast or _native()).batched(lhs, rhs, out, None if stream is None else stream.cuda_stream)
+    if r is not None:
+        return _checked(r)
     if lhs.dim() != 3 or rhs.dim() != 3:
         raise TTBError(f"batched_matmul expects rank-3 operands, got {lhs.dim()} and {rhs.dim()}")
     if lhs.device != rhs.device:
@@ -341,6 +370,9 @@ def batched_matmul_fused(lhs: torch.Tensor, rhs: torch.Tensor, addend: torch.Ten
     out += lhs . rhs).  Replaces the reference's matmul + expand + add (nn/linear.cpp:45-48),
     conv2d's per-image bias add (backend/cuda/conv.cu:163-183) and add_grad's second kernel
     (tensor/tensor.cpp:1137-1160)."""
+    r = (_fast or _native()).fused(lhs, rhs, addend, activation, out, None if stream is None else stream.cuda_stream)
+    if r is not None:
+        return _checked(r)
     if lhs.dim() != 3 or rhs.dim() != 3 or lhs.dtype != rhs.dtype or lhs.device != rhs.device:
         raise TTBError("operands must be rank-3 tensors of one dtype on one device")
     if lhs.device.type != "cuda":
@@ -379,6 +411,9 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor | None = No
            activation: Activation = Activation.NONE) -> torch.Tensor:
     """tinytensor's Linear.forward (nn/linear.cpp:41-50): x[..., in] . weight[in, out] + bias[out],
     as one fused kernel (the reference runs matmul, expand and a binary add)."""
+    r = (_fast or _native()).linear(x, weight, bias, activation)
+    if r is not None:
+        return _checked(r)
     if weight.dim() != 2 or x.shape[-1] != weight.shape[0]:
         raise TTBError(f"linear: x[..., {x.shape[-1]}] does not match weight {tuple(weight.shape)}")
     x2 = x.reshape(1, -1, x.shape[-1])
@@ -411,6 +446,9 @@ def conv2d(input: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor | None 
            padding: int = 0, stream=None) -> torch.Tensor:
     """tinytensor's conv2d forward (backend/cuda/conv.cu:37-197) through ``ttb_conv2d_forward``:
     input [B,C_in,H,W], weight [C_out,C_in,K,K], bias [C_out] -> [B,C_out,H_out,W_out]."""
+    r = (_fast or _native()).conv2d(input, weight, bias, stride, padding, None if stream is None else stream.cuda_stream)
+    if r is not None:
+        return _checked(r)
     d, oshape = _conv_desc(input, weight, stride, padding)
     input, weight = input.contiguous(), weight.contiguous()  # conv.cu:77
     if bias is not None:
@@ -433,6 +471,10 @@ def conv2d_backward(grad_output: torch.Tensor, input: torch.Tensor, weight: torc
                     padding: int = 0, with_bias: bool = True, stream=None):
     """conv2d backward (backend/cuda/conv.cu:199-403) through ``ttb_conv2d_backward``:
     -> (grad_input, grad_weight, grad_bias or None)."""
+    r = (_fast or _native()).conv2d_backward(grad_output, input, weight, stride, padding, with_bias,
+                                             None if stream is None else stream.cuda_stream)
+    if r is not None:
+        return _checked(r)
     d, oshape = _conv_desc(input, weight, stride, padding)
     if tuple(grad_output.shape) != tuple(oshape) or grad_output.dtype != input.dtype or grad_output.device != input.device:
         raise TTBError(f"conv2d backward: grad_output must be {tuple(oshape)} of the input's dtype and device")
@@ -594,6 +636,9 @@ def matmul(lhs: torch.Tensor, rhs: torch.Tensor) -> torch.Tensor:
     five rank forms funnelled into one rank-3 batched product.  No broadcasting of batch
     dims.  Unlike the reference, 2-D strided operands are passed as views (the reference's
     reshape clones them first, tensor.cpp:1386); the values are the same."""
+    r = (_fast or _native()).matmul(lhs, rhs)
+    if r is not None:
+        return _checked(r)
     if lhs.device != rhs.device:
         raise TTBError(f"Expected tensors to be on the same device. Given {lhs.device} and {rhs.device}")
     lhs, rhs = _promote(lhs, rhs)
@@ -638,6 +683,9 @@ def matmul_backward(lhs: torch.Tensor, rhs: torch.Tensor, grad_output: torch.Ten
     (autograd/binary_ops.cpp:172-179), i.e. two more products on PERMUTED VIEWS,
     ``grad . rhs^T`` and ``lhs^T . grad``, which go to the kernels uncopied.
     -> (grad_lhs, grad_rhs), shaped like the operands."""
+    r = (_fast or _native()).backward(lhs, rhs, grad_output)
+    if r is not None:
+        return _checked(r)
     ld, rd = lhs.dim(), rhs.dim()
     if (ld, rd) == (1, 1):
         l3, r3, g3 = lhs.reshape(1, 1, -1), rhs.reshape(1, -1, 1), grad_output.reshape(1, 1, 1)

@@ -48,6 +48,30 @@ HOST_SOURCES = ["generator.cpp"]
 HOST_FLAGS = ["-std=c++20", "-O3", "-DNDEBUG", "-march=x86-64-v3", "-fPIC", "-fvisibility=hidden", "-pthread"]
 
 
+# The native call path from torch tensors (csrc/torch_ext.cpp): a Python extension of its own, so that
+# libttb.so stays free of torch.
+EXT_SOURCE = "torch_ext.cpp"
+EXT = PKG / "_ttb_torch.so"
+
+
+def _build_ext() -> None:
+    import sysconfig
+
+    import torch
+    from torch.utils import cpp_extension
+
+    cuda_home = Path(_nvcc()).resolve().parent.parent
+    incs = [*cpp_extension.include_paths(), str(cuda_home / "include"), sysconfig.get_paths()["include"]]
+    lib_dir = Path(torch.__file__).resolve().parent / "lib"
+    cmd = [_cxx(), "-std=c++20", "-O2", "-DNDEBUG", "-fPIC", "-shared", "-fvisibility=hidden", "-w",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}", *(f"-I{i}" for i in incs),
+           str(CSRC / EXT_SOURCE), "-o", str(EXT), f"-L{lib_dir}", "-ltorch_python", "-ltorch", "-ltorch_cpu",
+           "-ltorch_cuda", "-lc10", "-lc10_cuda"]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError(f"compiling {EXT_SOURCE} failed:\n{r.stdout}\n{r.stderr}")
+
+
 def _cxx() -> str:
     exe = os.environ.get("CXX") or shutil.which("g++")
     if not exe:
@@ -102,6 +126,9 @@ def build(force: bool = False, verbose: bool = False) -> Path:
         r = subprocess.run(cmd, capture_output=True, text=True)
         if r.returncode != 0:
             raise RuntimeError(f"link failed:\n{r.stdout}\n{r.stderr}")
+    src_t = max((CSRC / EXT_SOURCE).stat().st_mtime, (PKG.parent / "include" / "ttb.h").stat().st_mtime)
+    if force or not EXT.exists() or EXT.stat().st_mtime < src_t:
+        _build_ext()
     if verbose:
         for name, log in logs.items():
             sys.stderr.write(f"==== {name}\n{log}\n")

@@ -1,0 +1,409 @@
+// torch_ext.cpp -- the call path from torch tensors to the C ABI, in native code.
+//
+// A product of a few microseconds is bound by the host: reading two tensors' shapes and strides
+// through Python, filling two ctypes structures and allocating the result took 15-25 us a call,
+// four times the launch itself.  These functions read the tensors' fields directly, allocate
+// the result and call the C ABI: host time of a 512 x 512 x 512 product 27 -> 9 us, of an x.W + b
+// and an accumulating h.W on 32 rows 80 -> 18 us, of the six products of an attention block
+// forward and backward 145 -> 29 us.
+//
+// Every function takes the ordinary case only (CUDA tensors of one supported dtype on one
+// device, shapes that fit) and returns None for anything else: the Python functions of the same
+// names then do the conversions or raise the error.  A status other than 0 comes back as an int.
+// The C ABI's entry points are handed over as addresses by bind(), so this module does not
+// link against libttb.so.
+#define PY_SSIZE_T_CLEAN
+#include <Python.h>
+
+#include <ATen/ATen.h>
+#include <ATen/cuda/EmptyTensor.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/autograd/python_variable.h>
+
+#include "../../include/ttb.h"
+
+namespace {
+
+decltype(&ttb_batched_matmul) p_matmul;
+decltype(&ttb_batched_matmul_strided_out) p_strided;
+decltype(&ttb_batched_matmul_fused) p_fused;
+decltype(&ttb_conv2d_forward) p_conv;
+decltype(&ttb_conv2d_backward) p_conv_bwd;
+
+int dtype_code(c10::ScalarType t) {
+    switch (t) {
+        case c10::ScalarType::Byte: return TTB_U8;
+        case c10::ScalarType::Short: return TTB_I16;
+        case c10::ScalarType::Int: return TTB_I32;
+        case c10::ScalarType::Long: return TTB_I64;
+        case c10::ScalarType::Float: return TTB_F32;
+        case c10::ScalarType::Double: return TTB_F64;
+        default: return 0;
+    }
+}
+
+const at::Tensor *tensor_of(PyObject *o) { return THPVariable_Check(o) ? &THPVariable_Unpack(o) : nullptr; }
+
+// Both are plain CUDA tensors with the same device and supported dtype.
+bool same_kind(const at::Tensor &a, const at::Tensor &b) {
+    return a.is_cuda() && b.is_cuda() && a.layout() == c10::kStrided && b.layout() == c10::kStrided &&
+           a.scalar_type() == b.scalar_type() && a.get_device() == b.get_device() && dtype_code(a.scalar_type()) != 0 &&
+           a.numel() > 0 && b.numel() > 0 && !a.is_conj() && !a.is_neg() && !b.is_neg();
+}
+
+ttb_view view3(const at::Tensor &t, int64_t s0, int64_t s1, int64_t s2, int64_t t0, int64_t t1, int64_t t2) {
+    ttb_view v;
+    v.data = t.const_data_ptr();
+    v.offset = 0;
+    v.size[0] = s0;
+    v.size[1] = s1;
+    v.size[2] = s2;
+    v.stride[0] = t0;
+    v.stride[1] = t1;
+    v.stride[2] = t2;
+    return v;
+}
+
+// A tensor of rank 2 or 3 as a rank-3 view; `transposed` exchanges the matrix dims.
+ttb_view view_of(const at::Tensor &t, bool transposed = false) {
+    const auto s = t.sizes(), st = t.strides();
+    const bool three = s.size() == 3;
+    const int r = three ? 1 : 0, c = r + 1;
+    const int64_t b = three ? s[0] : 1, bs = three ? st[0] : s[0] * s[1];
+    return transposed ? view3(t, b, s[c], s[r], bs, st[c], st[r]) : view3(t, b, s[r], s[c], bs, st[r], st[c]);
+}
+
+void *stream_for(int device, PyObject *stream) {
+    if (stream && stream != Py_None) {
+        return PyLong_AsVoidPtr(stream);
+    }
+    return c10::cuda::getCurrentCUDAStream(static_cast<c10::DeviceIndex>(device)).stream();
+}
+
+at::Tensor empty(at::IntArrayRef sizes, const at::Tensor &like) {
+    return at::detail::empty_cuda(sizes, like.scalar_type(), like.device(), std::nullopt);
+}
+
+PyObject *result(int rc, at::Tensor &&out) {
+    if (rc != TTB_OK) return PyLong_FromLong(rc);
+    return THPVariable_Wrap(std::move(out));
+}
+
+int call_matmul(const ttb_view &l, const ttb_view &r, void *out, int code, int dev, void *stream) {
+    int rc;
+    Py_BEGIN_ALLOW_THREADS rc = p_matmul(&l, &r, out, code, dev, stream);
+    Py_END_ALLOW_THREADS return rc;
+}
+
+// act(l . r + addend) -> out (contiguous, shaped `sizes`)
+int call_fused(const ttb_view &l, const ttb_view &r, void *out, const int64_t (&st)[3], const ttb_view *addend, int act,
+               int code, int dev, void *stream) {
+    int rc;
+    Py_BEGIN_ALLOW_THREADS rc = p_fused(&l, &r, out, 0, st, addend, act, code, dev, stream);
+    Py_END_ALLOW_THREADS return rc;
+}
+
+// The addend as a view of shape [B, N, M] by broadcasting rules; false when it does not expand.
+bool expand_view(const at::Tensor &t, int64_t B, int64_t N, int64_t M, ttb_view *v) {
+    const auto s = t.sizes(), st = t.strides();
+    const int64_t want[3] = {B, N, M};
+    if (s.size() > 3) return false;
+    int64_t stride[3] = {0, 0, 0};
+    for (int i = 0; i < static_cast<int>(s.size()); ++i) {
+        const int d = 3 - static_cast<int>(s.size()) + i;
+        if (s[i] == want[d])
+            stride[d] = want[d] == 1 ? 0 : st[i];
+        else if (s[i] != 1)
+            return false;
+    }
+    *v = view3(t, B, N, M, stride[0], stride[1], stride[2]);
+    return true;
+}
+
+#define TTB_TRY try {
+#define TTB_CATCH                                          \
+    }                                                      \
+    catch (const std::exception &e) {                      \
+        PyErr_SetString(PyExc_RuntimeError, e.what());     \
+        return nullptr;                                    \
+    }
+
+PyObject *py_bind(PyObject *, PyObject *const *a, Py_ssize_t n) {
+    if (n != 5) {
+        PyErr_SetString(PyExc_TypeError, "bind takes five addresses");
+        return nullptr;
+    }
+    p_matmul = reinterpret_cast<decltype(p_matmul)>(PyLong_AsVoidPtr(a[0]));
+    p_strided = reinterpret_cast<decltype(p_strided)>(PyLong_AsVoidPtr(a[1]));
+    p_fused = reinterpret_cast<decltype(p_fused)>(PyLong_AsVoidPtr(a[2]));
+    p_conv = reinterpret_cast<decltype(p_conv)>(PyLong_AsVoidPtr(a[3]));
+    p_conv_bwd = reinterpret_cast<decltype(p_conv_bwd)>(PyLong_AsVoidPtr(a[4]));
+    if (PyErr_Occurred()) return nullptr;
+    Py_RETURN_NONE;
+}
+
+// matmul(lhs, rhs): ranks 1.1, 1.2, 2.1, 2.2 and 3.3
+PyObject *py_matmul(PyObject *, PyObject *const *a, Py_ssize_t n) {
+    TTB_TRY;
+    if (n != 2) Py_RETURN_NONE;
+    const at::Tensor *lp = tensor_of(a[0]), *rp = tensor_of(a[1]);
+    if (!lp || !rp || !same_kind(*lp, *rp)) Py_RETURN_NONE;
+    const at::Tensor &l = *lp, &r = *rp;
+    const auto ls = l.sizes(), rs = r.sizes(), lt = l.strides(), rt = r.strides();
+    const int ld = static_cast<int>(ls.size()), rd = static_cast<int>(rs.size());
+    const int dev = l.get_device();
+    ttb_view lv, rv;
+    int64_t shape[3];
+    int rank;
+    if (ld == 2 && rd == 2) {
+        if (ls[1] != rs[0]) Py_RETURN_NONE;
+        lv = view_of(l), rv = view_of(r);
+        shape[0] = ls[0], shape[1] = rs[1], rank = 2;
+    } else if (ld == 3 && rd == 3) {
+        if (ls[2] != rs[1] || ls[0] != rs[0]) Py_RETURN_NONE;
+        lv = view_of(l), rv = view_of(r);
+        shape[0] = ls[0], shape[1] = ls[1], shape[2] = rs[2], rank = 3;
+    } else if (ld == 1 && rd == 2) {
+        if (ls[0] != rs[0]) Py_RETURN_NONE;
+        lv = view3(l, 1, 1, ls[0], ls[0], ls[0], lt[0]), rv = view_of(r);
+        shape[0] = rs[1], rank = 1;
+    } else if (ld == 2 && rd == 1) {
+        if (ls[1] != rs[0]) Py_RETURN_NONE;
+        lv = view_of(l), rv = view3(r, 1, rs[0], 1, rs[0], rt[0], 1);
+        shape[0] = ls[0], rank = 1;
+    } else if (ld == 1 && rd == 1) {
+        if (ls[0] != rs[0]) Py_RETURN_NONE;
+        lv = view3(l, 1, 1, ls[0], ls[0], ls[0], lt[0]), rv = view3(r, 1, rs[0], 1, rs[0], rt[0], 1);
+        shape[0] = 1, rank = 1;
+    } else {
+        Py_RETURN_NONE;
+    }
+    c10::cuda::OptionalCUDAGuard guard(l.device());
+    at::Tensor out = empty(at::IntArrayRef(shape, rank), l);
+    const int rc = call_matmul(lv, rv, out.mutable_data_ptr(), dtype_code(l.scalar_type()), dev, stream_for(dev, nullptr));
+    return result(rc, std::move(out));
+    TTB_CATCH;
+}
+
+// batched_matmul(lhs, rhs, out or None, stream pointer or None): rank 3
+PyObject *py_batched(PyObject *, PyObject *const *a, Py_ssize_t n) {
+    TTB_TRY;
+    if (n != 4) Py_RETURN_NONE;
+    const at::Tensor *lp = tensor_of(a[0]), *rp = tensor_of(a[1]);
+    if (!lp || !rp || !same_kind(*lp, *rp)) Py_RETURN_NONE;
+    const at::Tensor &l = *lp, &r = *rp;
+    if (l.dim() != 3 || r.dim() != 3 || l.size(2) != r.size(1) || l.size(0) != r.size(0)) Py_RETURN_NONE;
+    const int dev = l.get_device(), code = dtype_code(l.scalar_type());
+    void *stream = stream_for(dev, a[3]);
+    if (PyErr_Occurred()) return nullptr;
+    const ttb_view lv = view_of(l), rv = view_of(r);
+    if (a[2] == Py_None) {
+        c10::cuda::OptionalCUDAGuard guard(l.device());
+        at::Tensor out = empty({l.size(0), l.size(1), r.size(2)}, l);
+        const int rc = call_matmul(lv, rv, out.mutable_data_ptr(), code, dev, stream);
+        return result(rc, std::move(out));
+    }
+    const at::Tensor *op = tensor_of(a[2]);
+    if (!op || !same_kind(l, *op) || op->dim() != 3 || op->size(0) != l.size(0) || op->size(1) != l.size(1) ||
+        op->size(2) != r.size(2))
+        Py_RETURN_NONE;
+    const auto st = op->strides();
+    const int64_t strides[3] = {st[0], st[1], st[2]};
+    int rc;
+    void *dst = op->mutable_data_ptr();
+    Py_BEGIN_ALLOW_THREADS rc = p_strided(&lv, &rv, dst, 0, strides, code, dev, stream);
+    Py_END_ALLOW_THREADS if (rc != TTB_OK) return PyLong_FromLong(rc);
+    Py_INCREF(a[2]);
+    return a[2];
+    TTB_CATCH;
+}
+
+// fused(lhs, rhs, addend or None, activation, out or None, stream pointer or None): rank 3
+PyObject *py_fused(PyObject *, PyObject *const *a, Py_ssize_t n) {
+    TTB_TRY;
+    if (n != 6) Py_RETURN_NONE;
+    const at::Tensor *lp = tensor_of(a[0]), *rp = tensor_of(a[1]);
+    if (!lp || !rp || !same_kind(*lp, *rp)) Py_RETURN_NONE;
+    const at::Tensor &l = *lp, &r = *rp;
+    if (l.dim() != 3 || r.dim() != 3 || l.size(2) != r.size(1) || l.size(0) != r.size(0)) Py_RETURN_NONE;
+    const int64_t B = l.size(0), N = l.size(1), M = r.size(2);
+    const int dev = l.get_device(), code = dtype_code(l.scalar_type());
+    ttb_view av;
+    if (a[2] != Py_None) {
+        const at::Tensor *ap = tensor_of(a[2]);
+        if (!ap || !same_kind(l, *ap) || !expand_view(*ap, B, N, M, &av)) Py_RETURN_NONE;
+    }
+    const long act = PyLong_AsLong(a[3]);
+    void *stream = stream_for(dev, a[5]);
+    if (PyErr_Occurred()) return nullptr;
+    const ttb_view lv = view_of(l), rv = view_of(r);
+    if (a[4] == Py_None) {
+        c10::cuda::OptionalCUDAGuard guard(l.device());
+        at::Tensor out = empty({B, N, M}, l);
+        const int64_t strides[3] = {N * M, M, 1};
+        const int rc = call_fused(lv, rv, out.mutable_data_ptr(), strides, a[2] != Py_None ? &av : nullptr,
+                                  static_cast<int>(act), code, dev, stream);
+        return result(rc, std::move(out));
+    }
+    const at::Tensor *op = tensor_of(a[4]);
+    if (!op || !same_kind(l, *op) || op->dim() != 3 || op->size(0) != B || op->size(1) != N || op->size(2) != M)
+        Py_RETURN_NONE;
+    const auto st = op->strides();
+    const int64_t strides[3] = {st[0], st[1], st[2]};
+    const int rc = call_fused(lv, rv, op->mutable_data_ptr(), strides, a[2] != Py_None ? &av : nullptr,
+                              static_cast<int>(act), code, dev, stream);
+    if (rc != TTB_OK) return PyLong_FromLong(rc);
+    Py_INCREF(a[4]);
+    return a[4];
+    TTB_CATCH;
+}
+
+// linear(x[..., in], weight[in, out], bias[out] or None, activation); leading dims must be dense
+PyObject *py_linear(PyObject *, PyObject *const *a, Py_ssize_t n) {
+    TTB_TRY;
+    if (n != 4) Py_RETURN_NONE;
+    const at::Tensor *xp = tensor_of(a[0]), *wp = tensor_of(a[1]);
+    if (!xp || !wp || !same_kind(*xp, *wp)) Py_RETURN_NONE;
+    const at::Tensor &x = *xp, &w = *wp;
+    const int64_t xd = x.dim();
+    if (w.dim() != 2 || xd < 1 || xd > 8 || x.size(xd - 1) != w.size(0)) Py_RETURN_NONE;
+    if (xd != 2 && !x.is_contiguous()) Py_RETURN_NONE;
+    const int64_t K = w.size(0), M = w.size(1), N = x.numel() / K;
+    const int dev = x.get_device(), code = dtype_code(x.scalar_type());
+    ttb_view av;
+    if (a[2] != Py_None) {
+        const at::Tensor *bp = tensor_of(a[2]);
+        if (!bp || !same_kind(x, *bp) || !expand_view(*bp, 1, N, M, &av)) Py_RETURN_NONE;
+    }
+    const long act = PyLong_AsLong(a[3]);
+    if (PyErr_Occurred()) return nullptr;
+    const ttb_view xv = xd == 2 ? view_of(x) : view3(x, 1, N, K, N * K, K, 1), wv = view_of(w);
+    int64_t shape[8];
+    for (int64_t i = 0; i < xd - 1; ++i) shape[i] = x.size(i);
+    shape[xd - 1] = M;
+    c10::cuda::OptionalCUDAGuard guard(x.device());
+    at::Tensor out = empty(at::IntArrayRef(shape, static_cast<size_t>(xd)), x);
+    const int64_t strides[3] = {N * M, M, 1};
+    const int rc = call_fused(xv, wv, out.mutable_data_ptr(), strides, a[2] != Py_None ? &av : nullptr,
+                              static_cast<int>(act), code, dev, stream_for(dev, nullptr));
+    return result(rc, std::move(out));
+    TTB_CATCH;
+}
+
+// matmul_backward(lhs, rhs, grad): ranks 2.2 and 3.3 -> (grad . rhs^T, lhs^T . grad)
+PyObject *py_backward(PyObject *, PyObject *const *a, Py_ssize_t n) {
+    TTB_TRY;
+    if (n != 3) Py_RETURN_NONE;
+    const at::Tensor *lp = tensor_of(a[0]), *rp = tensor_of(a[1]), *gp = tensor_of(a[2]);
+    if (!lp || !rp || !gp || !same_kind(*lp, *rp) || !same_kind(*lp, *gp)) Py_RETURN_NONE;
+    const at::Tensor &l = *lp, &r = *rp, &g = *gp;
+    const int64_t d = l.dim();
+    if ((d != 2 && d != 3) || r.dim() != d || g.dim() != d) Py_RETURN_NONE;
+    if (d == 3 && (l.size(0) != r.size(0) || l.size(0) != g.size(0))) Py_RETURN_NONE;
+    if (l.size(d - 1) != r.size(d - 2) || g.size(d - 2) != l.size(d - 2) || g.size(d - 1) != r.size(d - 1)) Py_RETURN_NONE;
+    const int dev = l.get_device(), code = dtype_code(l.scalar_type());
+    void *stream = stream_for(dev, nullptr);
+    c10::cuda::OptionalCUDAGuard guard(l.device());
+    at::Tensor gl = empty(l.sizes(), l), gr = empty(r.sizes(), r);
+    int rc = call_matmul(view_of(g), view_of(r, true), gl.mutable_data_ptr(), code, dev, stream);
+    if (rc == TTB_OK) rc = call_matmul(view_of(l, true), view_of(g), gr.mutable_data_ptr(), code, dev, stream);
+    if (rc != TTB_OK) return PyLong_FromLong(rc);
+    PyObject *o0 = THPVariable_Wrap(std::move(gl)), *o1 = THPVariable_Wrap(std::move(gr));
+    PyObject *t = PyTuple_Pack(2, o0, o1);
+    Py_XDECREF(o0);
+    Py_XDECREF(o1);
+    return t;
+    TTB_CATCH;
+}
+
+// The description of a convolution of contiguous operands; false when it is not an ordinary one.
+bool conv_desc(const at::Tensor &x, const at::Tensor &w, PyObject *stride, PyObject *padding, ttb_conv2d_desc *d,
+               int64_t (&oshape)[4]) {
+    if (!same_kind(x, w) || x.dim() != 4 || w.dim() != 4 || x.size(1) != w.size(1) || w.size(2) != w.size(3) ||
+        !x.is_contiguous() || !w.is_contiguous())
+        return false;
+    const long S = PyLong_AsLong(stride), P = PyLong_AsLong(padding);
+    if (PyErr_Occurred()) {
+        PyErr_Clear();
+        return false;
+    }
+    const int64_t K = w.size(2);
+    if (S < 1 || P < 0 || x.size(2) + 2 * P < K || x.size(3) + 2 * P < K) return false;
+    *d = ttb_conv2d_desc{x.size(0), x.size(1), x.size(2), x.size(3), w.size(0), K, S, P};
+    oshape[0] = x.size(0);
+    oshape[1] = w.size(0);
+    oshape[2] = (x.size(2) + 2 * P - K) / S + 1;
+    oshape[3] = (x.size(3) + 2 * P - K) / S + 1;
+    return true;
+}
+
+// conv2d(input, weight, bias or None, stride, padding, stream pointer or None)
+PyObject *py_conv2d(PyObject *, PyObject *const *a, Py_ssize_t n) {
+    TTB_TRY;
+    if (n != 6) Py_RETURN_NONE;
+    const at::Tensor *xp = tensor_of(a[0]), *wp = tensor_of(a[1]), *bp = nullptr;
+    ttb_conv2d_desc d;
+    int64_t os[4];
+    if (!xp || !wp || !conv_desc(*xp, *wp, a[3], a[4], &d, os)) Py_RETURN_NONE;
+    if (a[2] != Py_None) {
+        bp = tensor_of(a[2]);
+        if (!bp || !same_kind(*xp, *bp) || bp->dim() != 1 || bp->size(0) != wp->size(0) || !bp->is_contiguous())
+            Py_RETURN_NONE;
+    }
+    const int dev = xp->get_device(), code = dtype_code(xp->scalar_type());
+    void *stream = stream_for(dev, a[5]);
+    if (PyErr_Occurred()) return nullptr;
+    c10::cuda::OptionalCUDAGuard guard(xp->device());
+    at::Tensor out = empty(os, *xp);
+    const void *x = xp->const_data_ptr(), *w = wp->const_data_ptr(), *b = bp ? bp->const_data_ptr() : nullptr;
+    void *o = out.mutable_data_ptr();
+    int rc;
+    Py_BEGIN_ALLOW_THREADS rc = p_conv(x, w, b, o, &d, code, dev, stream);
+    Py_END_ALLOW_THREADS return result(rc, std::move(out));
+    TTB_CATCH;
+}
+
+// conv2d_backward(grad_output, input, weight, stride, padding, with_bias, stream pointer or None)
+PyObject *py_conv2d_backward(PyObject *, PyObject *const *a, Py_ssize_t n) {
+    TTB_TRY;
+    if (n != 7) Py_RETURN_NONE;
+    const at::Tensor *gp = tensor_of(a[0]), *xp = tensor_of(a[1]), *wp = tensor_of(a[2]);
+    ttb_conv2d_desc d;
+    int64_t os[4];
+    if (!gp || !xp || !wp || !conv_desc(*xp, *wp, a[3], a[4], &d, os) || !same_kind(*xp, *gp) || !gp->is_contiguous() ||
+        gp->sizes() != at::IntArrayRef(os, 4))
+        Py_RETURN_NONE;
+    const int with_bias = PyObject_IsTrue(a[5]);
+    const int dev = xp->get_device(), code = dtype_code(xp->scalar_type());
+    void *stream = stream_for(dev, a[6]);
+    if (PyErr_Occurred()) return nullptr;
+    c10::cuda::OptionalCUDAGuard guard(xp->device());
+    at::Tensor gx = empty(xp->sizes(), *xp), gw = empty(wp->sizes(), *wp), gb;
+    if (with_bias) gb = empty({wp->size(0)}, *xp);
+    const void *g = gp->const_data_ptr(), *x = xp->const_data_ptr(), *w = wp->const_data_ptr();
+    void *ox = gx.mutable_data_ptr(), *ow = gw.mutable_data_ptr(), *ob = with_bias ? gb.mutable_data_ptr() : nullptr;
+    int rc;
+    Py_BEGIN_ALLOW_THREADS rc = p_conv_bwd(g, x, w, ox, ow, ob, &d, code, dev, stream);
+    Py_END_ALLOW_THREADS if (rc != TTB_OK) return PyLong_FromLong(rc);
+    PyObject *o0 = THPVariable_Wrap(std::move(gx)), *o1 = THPVariable_Wrap(std::move(gw));
+    PyObject *o2 = with_bias ? THPVariable_Wrap(std::move(gb)) : Py_NewRef(Py_None);
+    PyObject *t = PyTuple_Pack(3, o0, o1, o2);
+    Py_XDECREF(o0);
+    Py_XDECREF(o1);
+    Py_XDECREF(o2);
+    return t;
+    TTB_CATCH;
+}
+
+#define TTB_FAST(name, fn) {name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(fn)), METH_FASTCALL, nullptr}
+PyMethodDef methods[] = {TTB_FAST("bind", py_bind),         TTB_FAST("matmul", py_matmul),
+                         TTB_FAST("batched", py_batched),   TTB_FAST("fused", py_fused),
+                         TTB_FAST("linear", py_linear),     TTB_FAST("backward", py_backward),
+                         TTB_FAST("conv2d", py_conv2d),     TTB_FAST("conv2d_backward", py_conv2d_backward),
+                         {nullptr, nullptr, 0, nullptr}};
+PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "_ttb_torch", "torch tensors to the ttb C ABI", -1, methods};
+
+}  // namespace
+
+PyMODINIT_FUNC PyInit__ttb_torch(void) { return PyModule_Create(&module_def); }
