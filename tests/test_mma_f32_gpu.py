@@ -1,0 +1,121 @@
+"""The mma.sync f32 kernel and the padded copy in front of the tcgen05 kernel, at the edges: every
+tile and K split, both layouts of both operands, remainders in every dim, rows that start anywhere,
+Inf / NaN, and fused epilogues with a C whose rows are unaligned.  Gate: 1e-5 of the largest
+result, as for every f32 kernel (the split leaves 2^-19 per product)."""
+import numpy as np
+import pytest
+import torch
+
+from gpu_util import dev, host, rel_to_max
+
+pytestmark = pytest.mark.gpu
+F32_TOL = 1e-5
+
+
+@pytest.fixture
+def options(ttb, reset_options):
+    yield ttb
+    ttb.set_option("mma_tile", -1)
+    ttb.set_option("mma_splits", 0)
+
+
+def _operand(rng, shape, transposed, offset):
+    """A device view of `shape` whose storage starts `offset` elements in, stored as is or transposed."""
+    B, r, c = shape
+    stored = (B, c, r) if transposed else shape
+    base = torch.zeros(B * r * c + 8, device="cuda")
+    t = base[offset:offset + B * r * c].view(stored)
+    a = rng.standard_normal(shape).astype(np.float32)
+    t.copy_(dev(a.transpose(0, 2, 1) if transposed else a))
+    return a, (t.permute(0, 2, 1) if transposed else t)
+
+
+@pytest.mark.parametrize("tile", [0, 1, 2, 3, 4])
+@pytest.mark.parametrize("splits", [1, 2, 8])
+@pytest.mark.parametrize("shape", [(1, 1, 1, 1), (2, 33, 31, 17), (1, 65, 290, 63), (3, 129, 577, 66), (1, 64, 544, 128)])
+def test_tiles_splits_layouts(options, tile, splits, shape):
+    rng = np.random.default_rng(101)
+    B, N, K, M = shape
+    options.set_option("force_variant", int(options.Variant.MMA_F32))
+    options.set_option("mma_tile", tile)
+    options.set_option("mma_splits", splits)
+    for ta in (False, True):
+        for tb in (False, True):
+            for off in (0, 1):
+                a, A = _operand(rng, (B, N, K), ta, off)
+                b, Bm = _operand(rng, (B, K, M), tb, off)
+                got = host(options.batched_matmul(A, Bm))
+                assert options.last_variant() == options.Variant.MMA_F32
+                assert rel_to_max(got, np.matmul(a.astype(np.float64), b.astype(np.float64))) <= F32_TOL, (ta, tb, off)
+
+
+@pytest.mark.parametrize("shape", [(1, 300, 200, 270), (1, 48, 700, 10)])
+def test_non_finite(ttb, shape):
+    """Inf and NaN come out as an fp32 product gives them, and only where they belong."""
+    rng = np.random.default_rng(102)
+    B, N, K, M = shape
+    a = rng.standard_normal((B, N, K)).astype(np.float32)
+    b = rng.standard_normal((B, K, M)).astype(np.float32)
+    a[0, 5, 7], a[0, 9, 3], b[0, 11, 4] = np.inf, np.nan, -np.inf
+    got = host(ttb.batched_matmul(dev(a), dev(b)))
+    assert ttb.last_variant() in (ttb.Variant.MMA_F32, ttb.Variant.SIMT_SKINNY)
+    want = np.matmul(a.astype(np.float64), b.astype(np.float64))
+    assert np.array_equal(np.isnan(got), np.isnan(want))
+    assert np.array_equal(got[np.isinf(want)], want[np.isinf(want)].astype(np.float32))
+    fine = np.isfinite(want)
+    assert np.abs(got - want)[fine].max() / np.abs(want[fine]).max() <= F32_TOL
+
+
+@pytest.mark.parametrize("relu", [False, True])
+def test_fused_epilogue(options, relu):
+    rng = np.random.default_rng(103)
+    act = options.Activation.RELU if relu else options.Activation.NONE
+    for B, N, K, M in [(1, 37, 65, 131), (1, 200, 600, 70), (1, 90, 300, 12)]:
+        a, b = rng.standard_normal((B, N, K)).astype(np.float32), rng.standard_normal((B, K, M)).astype(np.float32)
+        for add in (rng.standard_normal(M), rng.standard_normal((N, 1)), rng.standard_normal((B, N, M))):
+            add = add.astype(np.float32)
+            want = np.matmul(a.astype(np.float64), b.astype(np.float64)) + add
+            want = np.maximum(want, 0) if relu else want
+            assert rel_to_max(host(options.batched_matmul_fused(dev(a), dev(b), dev(add), act)), want) <= F32_TOL
+        wide = torch.full((B, N, M + 3), 7.0, device="cuda")
+        options.batched_matmul(dev(a), dev(b), out=wide[:, :, 1:M + 1])
+        assert rel_to_max(host(wide[:, :, 1:M + 1]), np.matmul(a.astype(np.float64), b.astype(np.float64))) <= F32_TOL
+        assert (wide[:, :, 0] == 7).all() and (wide[:, :, M + 1:] == 7).all()
+
+
+@pytest.mark.parametrize("shape", [(1, 801, 1003, 769), (2, 515, 777, 901)])
+@pytest.mark.parametrize("layout", ["nn", "tn", "nt"])
+def test_padded_copy(ttb, shape, layout):
+    """Products too large for mma.sync whose rows TMA cannot describe."""
+    rng = np.random.default_rng(104)
+    B, N, K, M = shape
+    a, A = _operand(rng, (B, N, K), layout[0] == "t", 1)
+    b, Bm = _operand(rng, (B, K, M), layout[1] == "t", 3)
+    got = ttb.batched_matmul(A, Bm)
+    assert ttb.last_variant() in (ttb.Variant.TCGEN05_3XTF32, ttb.Variant.TCGEN05_2CTA)
+    want = np.matmul(a.astype(np.float64), b.astype(np.float64))
+    assert rel_to_max(host(got), want) <= F32_TOL
+    # one batch of A for all, and accumulation into C
+    C = got.clone()
+    ttb.batched_matmul_fused(A[:1].expand(B, N, K), Bm, C, out=C)
+    want = want + np.matmul(a[:1].astype(np.float64), b.astype(np.float64))
+    assert rel_to_max(host(C), want) <= F32_TOL
+
+
+def test_padded_copy_is_not_needed_in_a_capture(ttb):
+    """A capture on a stream without workspaces takes the kernel that needs none."""
+    rng = np.random.default_rng(105)
+    a, A = _operand(rng, (1, 801, 1003), False, 1)
+    b, Bm = _operand(rng, (1, 1003, 769), False, 1)
+    out = torch.zeros((1, 801, 769), device="cuda")
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.stream(side):
+        with torch.cuda.graph(graph, stream=side):
+            ttb.batched_matmul(A, Bm, out=out, stream=side)
+        assert ttb.last_variant() == ttb.Variant.MMA_F32
+        graph.replay()
+    torch.cuda.synchronize()
+    assert rel_to_max(host(out), np.matmul(a.astype(np.float64), b.astype(np.float64))) <= F32_TOL
+    ttb.check_device(0)

@@ -1,0 +1,47 @@
+"""The streaming kernels at the edges of their tiles: remainders of the four-element loads, of the
+K chunks and of the rows or columns of a block, one to sixteen tiny-dim entries, aligned and
+unaligned rows, with and without CTAs of a cluster sharing K.  Against the oracle / float64."""
+import numpy as np
+import pytest
+
+from gpu_util import dev, host, random_operands, rel_to_max
+
+pytestmark = pytest.mark.gpu
+
+# f32: a sum of K products in any order is within K * 2^-24 of sum |a||b|, far inside 1e-5 of the
+# largest result for the K here; f64 likewise with 2^-53.
+TOL = {np.dtype(np.float32): 1e-5, np.dtype(np.float64): 1e-12}
+
+
+def _check(ttb, oracle, A, B, a, b):
+    got = host(ttb.batched_matmul(A, B))
+    assert ttb.last_variant() == ttb.Variant.SIMT_SKINNY
+    if a.dtype.kind in "iu":
+        assert np.array_equal(got, oracle.matmul(a, b))
+    else:
+        wide = np.float64 if a.dtype == np.float32 else np.longdouble
+        assert rel_to_max(got, np.matmul(a.astype(wide), b.astype(wide))) <= TOL[a.dtype]
+
+
+@pytest.mark.parametrize("dt", [np.float32, np.float64, np.uint8, np.int64])
+@pytest.mark.parametrize("shape", [(1, 33, 64, 1), (2, 40, 67, 4), (1, 2501, 513, 9), (3, 2400, 256, 16), (1, 35, 730, 13)])
+def test_row_dot(ttb, oracle, dt, shape):
+    a, b = random_operands(np.random.default_rng(95), dt, *shape, -9, 10)
+    _check(ttb, oracle, dev(a), dev(b), a, b)
+
+
+@pytest.mark.parametrize("dt", [np.float32, np.float64, np.uint8, np.int64])
+@pytest.mark.parametrize("shape", [(1, 32, 64, 1), (2, 37, 130, 3), (1, 260, 1500, 1), (1, 515, 2049, 10), (1, 20000, 70, 16),
+                                   (5, 4100, 129, 7)])
+def test_col_stream(ttb, oracle, dt, shape):
+    B, N, K, M = shape
+    a, b = random_operands(np.random.default_rng(96), dt, *shape, -9, 10)
+    A = dev(np.ascontiguousarray(a.transpose(0, 2, 1))).permute(0, 2, 1)   # contiguous along its rows
+    _check(ttb, oracle, A, dev(b), a, b)
+
+
+@pytest.mark.parametrize("dt", [np.float32, np.float64, np.uint8, np.int64])
+@pytest.mark.parametrize("shape", [(1, 17, 1, 32), (2, 33, 4, 257), (1, 64, 5, 1024), (1, 31, 12, 130), (3, 100, 16, 515)])
+def test_outer(ttb, oracle, dt, shape):
+    a, b = random_operands(np.random.default_rng(97), dt, *shape, -9, 10)
+    _check(ttb, oracle, dev(a), dev(b), a, b)

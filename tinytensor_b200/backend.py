@@ -38,6 +38,7 @@ class Variant(enum.IntEnum):
     TCGEN05_2CTA = 5
     TCGEN05_I8LIMB = 6
     SIMT_SKINNY = 7
+    MMA_F32 = 8
 
 
 class _View(ctypes.Structure):

@@ -34,6 +34,8 @@ SOURCES = [
     "tma_desc.cu",
     "gemm_simt.cu",
     "gemm_f32_tcgen05.cu",
+    "gemm_f32_mma.cu",
+    "pack_f32.cu",
     "gemm_f64_dmma.cu",
     "gemm_i32_tcgen05.cu",
     "conv2d.cu",

@@ -98,12 +98,39 @@ struct F32Options {
 int launch_f32_tcgen05(const Problem &p, const F32Options &opt, int n_peers = 0, void *const *peer_c = nullptr,
                        void *mc_c = nullptr);
 bool f32_tcgen05_eligible(const Problem &p, char *why, int why_len);
+// tile: -1 = by shape, else 0 (128 x 16), 1 (32 x 64, K blocks halved over two groups of warps), 2 (64 x 64),
+// 3 (32 x 64), 4 (64 x 16, halved); splits of K over a cluster: 0 = by shape.
+int launch_f32_mma(const Problem &p, int tile = -1, int splits = 0);
+bool f32_mma_eligible(const Problem &p);
+// Copies operands that TMA cannot describe into padded rows (unit stride along one matrix dim needed).
+int pack_f32_operands(Problem *p);
 // two_cta: -1 = pick CTA pairs by shape, 0 = never, 1 = always.
 int launch_i32_tcgen05(const Problem &p, int two_cta = -1, int dbg = 0);
 bool i32_tcgen05_eligible(const Problem &p, char *why, int why_len);
 int launch_f64_dmma(const Problem &p);
 int measure_fp64_tensor_peak(int device, double *tflops);
 bool f64_dmma_eligible(const Problem &p);
+
+// out^T = rhs^T . lhs^T: the same product with the roles of the two operands (and of the
+// output's dims) exchanged, so that a tiny N is handled by the kernels written for a tiny M.
+inline Problem transposed(const Problem &p) {
+    Problem t = p;
+    t.a = p.b;
+    t.a_sb = p.b_sb;
+    t.a_si = p.b_sj;
+    t.a_sk = p.b_sk;
+    t.b = p.a;
+    t.b_sb = p.a_sb;
+    t.b_sk = p.a_sk;
+    t.b_sj = p.a_si;
+    t.N = p.M;
+    t.M = p.N;
+    t.c_si = p.c_sj;
+    t.c_sj = p.c_si;
+    t.d_si = p.d_sj;
+    t.d_sj = p.d_si;
+    return t;
+}
 
 size_t dtype_size(int dtype);
 

@@ -1,0 +1,569 @@
+// gemm_f32_mma.cu -- f32 batched GEMM on warp-level tensor-core instructions (mma.sync), for the
+// products whose time is latency and not arithmetic, and for views that TMA cannot describe.
+//
+// The tcgen05 kernel needs 6 us from its first load to its last store (TMA -> converter warps ->
+// tensor core -> tensor memory -> staged store) and fills an SM with one CTA, so a product of a
+// few K blocks spends its time in that chain; and it cannot take rows that are not 16-byte
+// aligned.  Here a CTA is a small tile with the whole split done in registers: cp.async brings
+// fp32 words (16 bytes each where the view is aligned, 4 bytes each for any other stride or
+// offset) into a ring of shared-memory stages, fragments are read, split and multiplied by the
+// same warp, two to four CTAs share an SM and hide each other's latency, and the CTAs of a
+// cluster split K when the tiles alone would leave SMs idle (sums meet through distributed
+// shared memory: one launch, no scratch, fixed order).
+//
+// Arithmetic: the hybrid split of the tcgen05 kernel (see gemm_f32_tcgen05.cu): x = big + small with
+// big = x truncated to TF32, A.B = big.big (TF32) + bf16(small_A).bf16(B) + bf16(A).bf16(small_B).  An
+// m16n8k16 bf16 fragment holds two k's per register where two m16n8k8 TF32 fragments hold k and
+// k + 4; any pairing of k's is right as long as A and B agree, so the bf16 fragments are packed from
+// the TF32 ones in place.  Non-finite elements are zero in the bf16 operands and travel through
+// the TF32 product alone.  The tensor core's accumulator does not round to nearest, so every 256
+// of K it is added into fp32 registers and restarted.
+//
+// Bounds: two TF32 and two bf16 instructions per 16 x 8 x 16, at the measured 275 and 550 TFLOP/s of
+// mma.sync, give 137 TFLOP/s; a large product reaches 62 (tensor pipe 45 % active: with 160 registers
+// a scheduler holds three warps, too few to hide the chain of reads, splits and MMAs), so large ones
+// go to the tcgen05 kernel.  Small ones, device time against that kernel and the CUDA-core one:
+// 32 x 128 x 512 9.7 -> 4.1 us, 512^3 19.7 -> 9.7-10.6, 64 x 2048 x 64 36.6 -> 7.4,
+// 500 x 333 x 201 25.0 -> 7.3, 4096 x 1024 x 10 15.9 -> 8.5.
+//
+// Replaces matmul_kernel<float> of the reference for these sizes and views
+// (tinytensor/tensor/backend/cuda/kernel/matmul.cuh:27-151).
+#include <cuda_bf16.h>
+
+#include <atomic>
+
+#include "common.cuh"
+
+namespace ttb {
+namespace {
+
+constexpr int BK = 32;
+constexpr int FOLD_KB = 8;  // K blocks between additions of the tensor core's sums into registers
+
+struct MmaArgs {
+    const float *a;
+    const float *b;
+    float *c;
+    int N, K, M;
+    long long a_sb, a_s, a_k;  // element strides: batch, row of A / column of B, K
+    long long b_sb, b_s, b_k;
+    long long c_sb, c_si, c_sj;
+    int a_vec, b_vec;  // 16-byte loads
+    int c_vec;         // rows of C start on a 16-byte boundary
+    int splits, k_per_split;
+    Epilogue ep;
+};
+
+__device__ __forceinline__ uint32_t smem_addr(const void *p) {
+    return static_cast<uint32_t>(__cvta_generic_to_shared(p));
+}
+// bytes < 16 (or < 4): the rest of the destination is zero-filled.
+__device__ __forceinline__ void cp16(uint32_t dst, const void *src, int bytes) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void cp4(uint32_t dst, const void *src, int bytes) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_wait() {
+    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+__device__ __forceinline__ uint32_t cluster_rank() {
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ const float *in_cta(const float *p, uint32_t rank) {
+    uint64_t out;
+    asm volatile("mapa.u64 %0, %1, %2;" : "=l"(out) : "l"(reinterpret_cast<uint64_t>(p)), "r"(rank));
+    return reinterpret_cast<const float *>(out);
+}
+
+__device__ __forceinline__ void mma_tf32(float (&c)[4], const uint32_t (&a)[4], const uint32_t (&b)[2]) {
+    asm volatile(
+        "mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
+}
+__device__ __forceinline__ void mma_bf16(float (&c)[4], const uint32_t (&a)[4], const uint32_t (&b)[2]) {
+    asm volatile(
+        "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
+}
+
+// Two fp32 words of one fragment position (k and k + 4): their TF32 parts, and bf16 pairs of the low
+// parts and of the values themselves.  `z` stays finite as long as every word seen is finite: the
+// low part of Inf and NaN is NaN, and NaN survives every multiply-add after it.
+__device__ __forceinline__ void split2(float x, float y, uint32_t &bx, uint32_t &by, uint32_t &s, uint32_t &v, float &z) {
+    bx = __float_as_uint(x) & 0xFFFFE000u;
+    by = __float_as_uint(y) & 0xFFFFE000u;
+    const float dx = x - __uint_as_float(bx), dy = y - __uint_as_float(by);
+    const __nv_bfloat162 p = __floats2bfloat162_rn(dx, dy);
+    const __nv_bfloat162 q = __floats2bfloat162_rn(x, y);
+    z = fmaf(dx, dy, z);
+    s = *reinterpret_cast<const uint32_t *>(&p);
+    v = *reinterpret_cast<const uint32_t *>(&q);
+}
+// Zeroes the bf16 entries whose low part is NaN, that is, those of Inf and NaN.
+__device__ __forceinline__ void keep_finite(uint32_t &s, uint32_t &v) {
+    const __nv_bfloat162 p = *reinterpret_cast<const __nv_bfloat162 *>(&s);
+    const uint32_t keep = __heq2_mask(p, p);
+    s &= keep;
+    v &= keep;
+}
+// Four 8 x 4 blocks of fp32 words, one word per thread of each: row (lane / 4), word (lane % 4) of the
+// block whose row r starts at the address lane 8 * block + r passes.
+__device__ __forceinline__ void ldmatrix4(uint32_t (&v)[4], uint32_t addr) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3])
+                 : "r"(addr)
+                 : "memory");
+}
+
+// Brings BK-deep slices of an operand tile of ROWS rows (A) or columns (B) into shared memory:
+// [row][k] with a pitch of BK + 4 words, or, for an operand contiguous along its rows (MN),
+// [k][row] with a pitch of ROWS + 8: both make the fragment reads conflict-free.  A thread's
+// pieces lie `step` apart in memory and a constant apart in shared memory, in K (MN) or along the
+// rows, so that a piece costs an addition, a comparison and the copy.
+template <int ROWS, bool MN, int THREADS>
+struct Loader {
+    static constexpr int PITCH = MN ? ROWS + 8 : BK + 4;
+    const float *p;        // this thread's first piece of the next slice
+    long long step;        // elements from piece to piece
+    long long slice_step;  // elements from slice to slice
+    uint32_t dst;          // byte offset of the first piece in the slice
+    int left;              // rows left from this thread's first one (not MN), or of them loaded by a piece (MN)
+    int k;                 // first k of this thread within a slice
+    bool vec;
+
+    __device__ Loader(const float *src, long long s_row, long long s_k, int row0, int rows, int k0, bool vec_) : vec(vec_) {
+        const int wide = vec ? 4 : 1;
+        const int across = (MN ? ROWS : BK) / wide;  // pieces side by side
+        const int x = static_cast<int>(threadIdx.x) % across * wide, y = static_cast<int>(threadIdx.x) / across;
+        const int r = MN ? x : y;
+        k = MN ? y : x;
+        p = src + (row0 + r) * s_row + (k0 + k) * s_k;
+        step = (THREADS / across) * (MN ? s_k : s_row);
+        slice_step = BK * s_k;
+        dst = static_cast<uint32_t>((MN ? k * PITCH + r : r * PITCH + k) * 4);
+        left = rows - row0 - r;
+    }
+    // The next slice, of which k_left k's exist.
+    __device__ __forceinline__ void load(uint32_t slice, int k_left) {
+        k_left -= k;
+        const uint32_t to = slice + dst;
+        if (vec) {
+            constexpr int ACROSS = (MN ? ROWS : BK) / 4, DOWN = THREADS / ACROSS, N = (MN ? BK : ROWS);
+            const int words = MN ? left : k_left;  // of the 4 of a piece
+            const int bytes = words >= 4 ? 16 : (words > 0 ? words * 4 : 0);
+            const int lines = MN ? k_left : left;
+            const float *from = p;
+#pragma unroll
+            for (int i = 0; i < (N + DOWN - 1) / DOWN; ++i) {
+                if (N % DOWN != 0 && static_cast<int>(threadIdx.x) / ACROSS + i * DOWN >= N) break;
+                cp16(to + i * DOWN * PITCH * 4, from, i * DOWN < lines ? bytes : 0);
+                from += step;
+            }
+        } else {
+            constexpr int ACROSS = MN ? ROWS : BK, DOWN = THREADS / ACROSS, N = (MN ? BK : ROWS);
+            const bool in = (MN ? left : k_left) > 0;
+            const int lines = MN ? k_left : left;
+            const float *from = p;
+#pragma unroll
+            for (int i = 0; i < N / DOWN; ++i) {
+                cp4(to + i * DOWN * PITCH * 4, from, in && i * DOWN < lines ? 4 : 0);
+                from += step;
+            }
+        }
+        p += slice_step;
+    }
+};
+
+__device__ __forceinline__ float finish(float v, const Epilogue &ep, long long b, int i, int j) {
+    if (ep.d) v += static_cast<const float *>(ep.d)[b * ep.d_sb + i * ep.d_si + j * ep.d_sj];
+    if (ep.act == TTB_ACT_RELU) v = v < 0.0f ? 0.0f : v;
+    return v;
+}
+
+template <int BM, int BN, int WARPS_M, int WARPS_N, int WARPS_K, int STAGES, bool A_MN, bool B_MN>
+struct Tile {
+    static constexpr int THREADS = WARPS_M * WARPS_N * WARPS_K * 32;
+    static constexpr int A_WORDS = A_MN ? BK * (BM + 8) : BM * (BK + 4);
+    static constexpr int STAGE_WORDS = A_WORDS + (B_MN ? BK * (BN + 8) : BN * (BK + 4));
+    static constexpr int RING = STAGES * STAGE_WORDS, SUMS = BM * (BN + 4);
+    static constexpr int SMEM = (RING > SUMS ? RING : SUMS) * 4;
+};
+
+// WARPS_K = 2: two groups of warps take a K block's halves (their sums meet in shared memory at
+// the end), which halves the time a small product waits for one warp's chain of reads, splits and
+// MMAs.
+template <int BM, int BN, int WARPS_M, int WARPS_N, int WARPS_K, int STAGES, int MIN_CTAS, bool A_MN, bool B_MN>
+__global__ void __launch_bounds__(WARPS_M *WARPS_N *WARPS_K * 32, MIN_CTAS) gemm_f32_mma_kernel(const MmaArgs p) {
+    using T = Tile<BM, BN, WARPS_M, WARPS_N, WARPS_K, STAGES, A_MN, B_MN>;
+    constexpr int THREADS = T::THREADS;
+    constexpr int WM = BM / WARPS_M, WN = BN / WARPS_N, MI = WM / 16, NI = WN / 8;
+    constexpr int PA = A_MN ? BM + 8 : BK + 4, PB = B_MN ? BN + 8 : BK + 4;
+    constexpr int A_WORDS = T::A_WORDS, STAGE_WORDS = T::STAGE_WORDS;
+    extern __shared__ __align__(16) float smem[];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int g = lane >> 2, t = lane & 3;
+    const int wk = warp / (WARPS_M * WARPS_N);  // which half of a K block (WARPS_K == 2)
+    const int wm = (warp / WARPS_N) % WARPS_M * WM, wn = (warp % WARPS_N) * WN;
+    const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
+    const long long batch = blockIdx.z / p.splits;
+    const int split = blockIdx.z % p.splits;
+    const int k_begin = split * p.k_per_split;
+    const int k_end = k_begin + p.k_per_split < p.K ? k_begin + p.k_per_split : p.K;
+    const float *a = p.a + batch * p.a_sb, *b = p.b + batch * p.b_sb;
+    const uint32_t ring = smem_addr(smem);
+
+    Loader<BM, A_MN, THREADS> load_a(a, p.a_s, p.a_k, m0, p.N, k_begin, p.a_vec != 0);
+    Loader<BN, B_MN, THREADS> load_b(b, p.b_s, p.b_k, n0, p.M, k_begin, p.b_vec != 0);
+    int k_left = k_end - k_begin;  // K not yet asked for
+    auto load = [&](int stage) {
+        const uint32_t dst = ring + stage * (STAGE_WORDS * 4);
+        load_a.load(dst, k_left);
+        load_b.load(dst + A_WORDS * 4, k_left);
+        k_left -= BK;
+    };
+
+    float acc[MI][NI][4], sum[MI][NI][4];
+#pragma unroll
+    for (int i = 0; i < MI; ++i)
+#pragma unroll
+        for (int j = 0; j < NI; ++j)
+#pragma unroll
+            for (int r = 0; r < 4; ++r) acc[i][j][r] = sum[i][j][r] = 0.0f;
+
+    const int num_kb = k_end > k_begin ? (k_end - k_begin + BK - 1) / BK : 0;
+#pragma unroll
+    for (int s = 0; s < STAGES - 1; ++s) {
+        if (s < num_kb) load(s);
+        cp_commit();
+    }
+    int stage = 0;
+    for (int kb = 0; kb < num_kb; ++kb) {
+        cp_wait<STAGES - 2>();
+        __syncthreads();
+        if (k_left > 0) load(stage == 0 ? STAGES - 1 : stage - 1);
+        cp_commit();
+        const float *as = smem + stage * STAGE_WORDS, *bs = as + A_WORDS;
+        const uint32_t as32 = ring + stage * (STAGE_WORDS * 4), bs32 = as32 + A_WORDS * 4;
+        if (++stage == STAGES) stage = 0;
+#pragma unroll
+        for (int k1 = 0; k1 < BK / WARPS_K; k1 += 16) {
+            const int k = WARPS_K == 2 ? wk * 16 : k1;
+            uint32_t a_big[MI][2][4], a_low[MI][4], a_val[MI][4];
+            uint32_t b_big[NI][2][2], b_low[NI][2], b_val[NI][2];
+            float z = 0.0f;
+#pragma unroll
+            for (int j = 0; j < NI; ++j) {
+                // words (k + t, k + t + 4, k + 8 + t, k + 12 + t) of column g
+                uint32_t w[4];
+                if constexpr (B_MN) {
+                    const float *src = bs + (k + t) * PB + wn + j * 8 + g;
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) w[u] = __float_as_uint(src[u * 4 * PB]);
+                } else {
+                    ldmatrix4(w, bs32 + ((wn + j * 8 + (lane & 7)) * PB + k + (lane >> 3) * 4) * 4);
+                }
+#pragma unroll
+                for (int h = 0; h < 2; ++h)
+                    split2(__uint_as_float(w[2 * h]), __uint_as_float(w[2 * h + 1]), b_big[j][h][0], b_big[j][h][1],
+                           b_low[j][h], b_val[j][h], z);
+            }
+#pragma unroll
+            for (int i = 0; i < MI; ++i)
+#pragma unroll
+                for (int u = 0; u < 2; ++u) {
+                    // the same words of row g + 8 u
+                    uint32_t w[4];
+                    if constexpr (A_MN) {
+                        const float *src = as + (k + t) * PA + wm + i * 16 + u * 8 + g;
+#pragma unroll
+                        for (int q = 0; q < 4; ++q) w[q] = __float_as_uint(src[q * 4 * PA]);
+                    } else {
+                        ldmatrix4(w, as32 + ((wm + i * 16 + u * 8 + (lane & 7)) * PA + k + (lane >> 3) * 4) * 4);
+                    }
+#pragma unroll
+                    for (int h = 0; h < 2; ++h)
+                        split2(__uint_as_float(w[2 * h]), __uint_as_float(w[2 * h + 1]), a_big[i][h][u], a_big[i][h][u + 2],
+                               a_low[i][h * 2 + u], a_val[i][h * 2 + u], z);
+                }
+            if (!(fabsf(z) <= 3.0e38f)) {
+#pragma unroll
+                for (int j = 0; j < NI; ++j)
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) keep_finite(b_low[j][h], b_val[j][h]);
+#pragma unroll
+                for (int i = 0; i < MI; ++i)
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) keep_finite(a_low[i][q], a_val[i][q]);
+            }
+            __syncwarp();
+            // (one kind at a time over all tiles: a tile's next instruction comes MI x NI later)
+#pragma unroll
+            for (int i = 0; i < MI; ++i)
+#pragma unroll
+                for (int j = 0; j < NI; ++j) mma_bf16(acc[i][j], a_low[i], b_val[j]);
+#pragma unroll
+            for (int i = 0; i < MI; ++i)
+#pragma unroll
+                for (int j = 0; j < NI; ++j) mma_bf16(acc[i][j], a_val[i], b_low[j]);
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+#pragma unroll
+                for (int i = 0; i < MI; ++i)
+#pragma unroll
+                    for (int j = 0; j < NI; ++j) mma_tf32(acc[i][j], a_big[i][h], b_big[j][h]);
+        }
+        if ((kb & (FOLD_KB - 1)) == FOLD_KB - 1) {
+#pragma unroll
+            for (int i = 0; i < MI; ++i)
+#pragma unroll
+                for (int j = 0; j < NI; ++j)
+#pragma unroll
+                    for (int r = 0; r < 4; ++r) {
+                        sum[i][j][r] += acc[i][j][r];
+                        acc[i][j][r] = 0.0f;
+                    }
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < MI; ++i)
+#pragma unroll
+        for (int j = 0; j < NI; ++j)
+#pragma unroll
+            for (int r = 0; r < 4; ++r) sum[i][j][r] += acc[i][j][r];
+
+    constexpr int PS = BN + 4;
+    auto leave_sums = [&]() {
+#pragma unroll
+        for (int i = 0; i < MI; ++i)
+#pragma unroll
+            for (int j = 0; j < NI; ++j)
+#pragma unroll
+                for (int u = 0; u < 2; ++u)
+                    *reinterpret_cast<float2 *>(&smem[(wm + i * 16 + g + u * 8) * PS + wn + j * 8 + 2 * t]) =
+                        make_float2(sum[i][j][2 * u], sum[i][j][2 * u + 1]);
+    };
+    if constexpr (WARPS_K == 2) {
+        cp_wait<0>();
+        __syncthreads();
+        if (wk == 1) leave_sums();
+        __syncthreads();
+        if (wk == 0) {
+#pragma unroll
+            for (int i = 0; i < MI; ++i)
+#pragma unroll
+                for (int j = 0; j < NI; ++j)
+#pragma unroll
+                    for (int u = 0; u < 2; ++u) {
+                        const float2 v =
+                            *reinterpret_cast<const float2 *>(&smem[(wm + i * 16 + g + u * 8) * PS + wn + j * 8 + 2 * t]);
+                        sum[i][j][2 * u] += v.x;
+                        sum[i][j][2 * u + 1] += v.y;
+                    }
+        }
+    }
+    float *c = p.c + batch * p.c_sb;
+    if (p.splits == 1) {
+        if (WARPS_K == 2 && wk == 1) return;
+        // registers (row g / g + 8, columns 2t, 2t + 1) straight to C
+#pragma unroll
+        for (int i = 0; i < MI; ++i)
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                const int row = m0 + wm + i * 16 + g + u * 8;
+                if (row >= p.N) continue;
+                float *crow = c + row * p.c_si;
+#pragma unroll
+                for (int j = 0; j < NI; ++j) {
+                    const int col = n0 + wn + j * 8 + 2 * t;
+                    if (col >= p.M) continue;
+                    const float v0 = finish(sum[i][j][2 * u], p.ep, batch, row, col);
+                    if (col + 1 < p.M) {
+                        const float v1 = finish(sum[i][j][2 * u + 1], p.ep, batch, row, col + 1);
+                        if (p.c_vec) {
+                            *reinterpret_cast<float2 *>(crow + col) = make_float2(v0, v1);
+                        } else {
+                            crow[col * p.c_sj] = v0;
+                            crow[(col + 1) * p.c_sj] = v1;
+                        }
+                    } else {
+                        crow[col * p.c_sj] = v0;
+                    }
+                }
+            }
+        return;
+    }
+    // Sums of the cluster's CTAs: each leaves its tile in shared memory, CTA r finishes rows
+    // [r, r + 1) * BM / splits of it.
+    if constexpr (WARPS_K == 1) {
+        cp_wait<0>();
+        __syncthreads();
+    }
+    if (WARPS_K == 1 || wk == 0) leave_sums();
+    cluster_sync();
+    const int rows = BM / p.splits, r0 = static_cast<int>(cluster_rank()) * rows;
+    for (int idx = threadIdx.x; idx < rows * (BN / 4); idx += THREADS) {
+        const int r = r0 + idx / (BN / 4), cc = (idx % (BN / 4)) * 4;
+        const int row = m0 + r, col = n0 + cc;
+        if (row >= p.N || col >= p.M) continue;
+        float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        for (int q = 0; q < p.splits; ++q) {
+            const float4 w = *reinterpret_cast<const float4 *>(in_cta(&smem[r * PS + cc], static_cast<uint32_t>(q)));
+            v.x += w.x;
+            v.y += w.y;
+            v.z += w.z;
+            v.w += w.w;
+        }
+        float *dst = c + row * p.c_si + col * p.c_sj;
+        v.x = finish(v.x, p.ep, batch, row, col);
+        if (col + 1 < p.M) v.y = finish(v.y, p.ep, batch, row, col + 1);
+        if (col + 2 < p.M) v.z = finish(v.z, p.ep, batch, row, col + 2);
+        if (col + 3 < p.M) v.w = finish(v.w, p.ep, batch, row, col + 3);
+        if (p.c_vec && col + 4 <= p.M) {
+            *reinterpret_cast<float4 *>(dst) = v;
+        } else {
+            dst[0] = v.x;
+            if (col + 1 < p.M) dst[p.c_sj] = v.y;
+            if (col + 2 < p.M) dst[2 * p.c_sj] = v.z;
+            if (col + 3 < p.M) dst[3 * p.c_sj] = v.w;
+        }
+    }
+    cluster_sync();  // nobody leaves while its sums are being read
+}
+
+template <int BM, int BN, int WARPS_M, int WARPS_N, int WARPS_K, int STAGES, int MIN_CTAS, bool A_MN, bool B_MN>
+int launch_tile(const Problem &p, MmaArgs &args, int splits) {
+    using T = Tile<BM, BN, WARPS_M, WARPS_N, WARPS_K, STAGES, A_MN, B_MN>;
+    constexpr int bytes = T::SMEM;
+    auto kernel = gemm_f32_mma_kernel<BM, BN, WARPS_M, WARPS_N, WARPS_K, STAGES, MIN_CTAS, A_MN, B_MN>;
+    if (bytes > 48 * 1024) {
+        static std::atomic<bool> ready[64];
+        if (!ready[p.device & 63].load(std::memory_order_acquire)) {
+            cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+            if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute(smem)");
+            ready[p.device & 63].store(true, std::memory_order_release);
+        }
+    }
+    args.splits = splits;
+    const int kb = (args.K + BK - 1) / BK;
+    args.k_per_split = (kb + splits - 1) / splits * BK;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(static_cast<unsigned>((p.M + BN - 1) / BN), static_cast<unsigned>((p.N + BM - 1) / BM),
+                       static_cast<unsigned>(p.B * splits));
+    cfg.blockDim = dim3(T::THREADS);
+    cfg.dynamicSmemBytes = bytes;
+    cfg.stream = p.stream;
+    cudaLaunchAttribute attr[1];
+    if (splits > 1) {
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = 1;
+        attr[0].val.clusterDim.y = 1;
+        attr[0].val.clusterDim.z = static_cast<unsigned>(splits);
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+    }
+    cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, args);
+    return e == cudaSuccess ? TTB_OK : cuda_fail(e, "gemm_f32_mma_kernel launch");
+}
+
+template <int BM, int BN, int WARPS_M, int WARPS_N, int WARPS_K, int STAGES, int MIN_CTAS>
+int launch_layout(const Problem &p, MmaArgs &args, int splits, bool a_mn, bool b_mn) {
+    if (a_mn)
+        return b_mn ? launch_tile<BM, BN, WARPS_M, WARPS_N, WARPS_K, STAGES, MIN_CTAS, true, true>(p, args, splits)
+                    : launch_tile<BM, BN, WARPS_M, WARPS_N, WARPS_K, STAGES, MIN_CTAS, true, false>(p, args, splits);
+    return b_mn ? launch_tile<BM, BN, WARPS_M, WARPS_N, WARPS_K, STAGES, MIN_CTAS, false, true>(p, args, splits)
+                : launch_tile<BM, BN, WARPS_M, WARPS_N, WARPS_K, STAGES, MIN_CTAS, false, false>(p, args, splits);
+}
+
+// The row dim is contiguous, or nearer to it than K is.
+bool mn_major(long long s_row, long long s_k, long long rows, long long k) {
+    if (s_k == 1 && k > 1) return false;
+    if (s_row == 1 && rows > 1) return true;
+    return s_row < s_k;
+}
+// 16-byte loads: unit stride along the loaded dim, everything else a multiple of 16 bytes.
+bool vec_ok(const void *ptr, long long unit, long long other, long long batch) {
+    return unit == 1 && (other & 3) == 0 && (batch & 3) == 0 && (reinterpret_cast<uintptr_t>(ptr) & 15) == 0;
+}
+
+}  // namespace
+
+bool f32_mma_eligible(const Problem &p) {
+    // Unit stride along a matrix dim (any other gap wastes most of every sector read); 32-bit extents
+    // inside the kernel, and the launch limits of grid.y and grid.z (8 splits).
+    const bool a_unit = p.a_sk == 1 || p.a_si == 1 || p.K == 1 || p.N == 1;
+    const bool b_unit = p.b_sk == 1 || p.b_sj == 1 || p.K == 1 || p.M == 1;
+    return p.dtype == TTB_F32 && a_unit && b_unit && p.N <= 0x3FFFFFFF && p.M <= 0x3FFFFFFF && p.K <= 0x3FFFFFFF && p.B * 8 <= 65535 &&
+           (p.N + 31) / 32 <= 65535;
+}
+
+int launch_f32_mma(const Problem &p, int tile, int splits) {
+    if (!f32_mma_eligible(p)) {
+        set_error("mma.sync f32 kernel: extents beyond its launch limits");
+        return TTB_EUNSUPPORTED;
+    }
+    int sms = 148;
+    sm_count(p.device, &sms);
+    MmaArgs args{};
+    args.a = static_cast<const float *>(p.a);
+    args.b = static_cast<const float *>(p.b);
+    args.c = static_cast<float *>(p.c);
+    args.N = static_cast<int>(p.N);
+    args.K = static_cast<int>(p.K);
+    args.M = static_cast<int>(p.M);
+    args.a_sb = p.a_sb;
+    args.a_s = p.a_si;
+    args.a_k = p.a_sk;
+    args.b_sb = p.b_sb;
+    args.b_s = p.b_sj;
+    args.b_k = p.b_sk;
+    args.c_sb = p.c_sb;
+    args.c_si = p.c_si;
+    args.c_sj = p.c_sj;
+    args.ep = epilogue_of(p);
+    const bool a_mn = mn_major(p.a_si, p.a_sk, p.N, p.K), b_mn = mn_major(p.b_sj, p.b_sk, p.M, p.K);
+    args.a_vec = a_mn ? vec_ok(p.a, p.a_si, p.a_sk, p.a_sb) : vec_ok(p.a, p.a_sk, p.a_si, p.a_sb);
+    args.b_vec = b_mn ? vec_ok(p.b, p.b_sj, p.b_sk, p.b_sb) : vec_ok(p.b, p.b_sk, p.b_sj, p.b_sb);
+    args.c_vec = vec_ok(p.c, p.c_sj, p.c_si, p.c_sb);
+    auto tiles = [&](long long bm, long long bn) { return ((p.N + bm - 1) / bm) * ((p.M + bn - 1) / bn) * p.B; };
+    const int kb = (args.K + BK - 1) / BK;
+    // 32 x 64 tiles while 64 x 64 ones would fill less than a quarter of the SMs, with the K block cut
+    // over two groups of warps unless there are enough CTAs to hide each other's latency.
+    if (tile < 0) {
+        if (p.M <= 16)
+            tile = tiles(128, 16) * 8 < sms ? 4 : 0;
+        else if (p.N <= 32 || tiles(64, 64) < sms / 4)
+            tile = tiles(32, 64) >= 2LL * sms ? 3 : 1;
+        else
+            tile = 2;
+    }
+    const long long n = tile == 0   ? tiles(128, 16)
+                        : tile == 2 ? tiles(64, 64)
+                        : tile == 4 ? tiles(64, 16)
+                                    : tiles(32, 64);
+    if (splits <= 0) {
+        // CTAs along K until there are two per SM, while each keeps three K blocks: a cluster's
+        // exchange of sums costs about as much as one (512^3: 64 tiles x 4, 9.7-10.6 us; x 2, 12.0;
+        // not split, 13.4).
+        splits = 1;
+        while (splits < 8 && n * splits <= sms && kb >= 5 * splits) splits *= 2;
+    }
+    switch (tile) {
+        case 0: return launch_layout<128, 16, 4, 1, 1, 4, 2>(p, args, splits, a_mn, b_mn);
+        case 1: return launch_layout<32, 64, 2, 2, 2, 4, 2>(p, args, splits, a_mn, b_mn);
+        case 2: return launch_layout<64, 64, 2, 2, 1, 4, 3>(p, args, splits, a_mn, b_mn);
+        case 3: return launch_layout<32, 64, 2, 2, 1, 4, 4>(p, args, splits, a_mn, b_mn);
+        default: return launch_layout<64, 16, 4, 1, 2, 4, 2>(p, args, splits, a_mn, b_mn);
+    }
+}
+
+}  // namespace ttb

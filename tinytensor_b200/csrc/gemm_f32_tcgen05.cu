@@ -913,16 +913,24 @@ __global__ void __launch_bounds__(Cfg<CG>::NUM_THREADS, 1) gemm_f32_3xtf32_kerne
                 tc_fence_after_sync();
                 const uint32_t t_row = tmem_base + static_cast<uint32_t>(acc * C::ACC_COLS + col_half * 128) +
                                        (static_cast<uint32_t>(quarter * 32) << 16);
-                const bool first = ch == kb0;
+                if (ch == kb0) {
+                    // the first chunk of a tile is the sum so far: one wait for all 128 columns
+                    uint32_t v[4][32];
 #pragma unroll
-                for (int q = 0; q < 8; ++q) {
-                    uint32_t v[16];
-                    tmem_ld_32x16(t_row + static_cast<uint32_t>(q * 16), v);
+                    for (int q = 0; q < 4; ++q) tmem_ld_32x32(t_row + static_cast<uint32_t>(q * 32), v[q]);
                     tmem_ld_wait();
 #pragma unroll
-                    for (int j = 0; j < 16; ++j) {
-                        const float x = __uint_as_float(v[j]);
-                        sum[q * 16 + j] = first ? x : sum[q * 16 + j] + x;
+                    for (int q = 0; q < 4; ++q)
+#pragma unroll
+                        for (int j = 0; j < 32; ++j) sum[q * 32 + j] = __uint_as_float(v[q][j]);
+                } else {
+#pragma unroll
+                    for (int q = 0; q < 8; ++q) {
+                        uint32_t v[16];
+                        tmem_ld_32x16(t_row + static_cast<uint32_t>(q * 16), v);
+                        tmem_ld_wait();
+#pragma unroll
+                        for (int j = 0; j < 16; ++j) sum[q * 16 + j] += __uint_as_float(v[j]);
                     }
                 }
                 tc_fence_before_sync();
@@ -1197,13 +1205,23 @@ __global__ void __launch_bounds__(Cfg<CG>::NUM_THREADS, 1) gemm_f32_3xtf32_kerne
                     // (16-byte chunk XOR row) of a 32 x 32 TMA box, and one lane issues a bulk
                     // tensor store.  The copy engine writes whole lines and clips the box at the
                     // edges of C; the warp's LSU work is eight 16-byte shared stores per chunk.
-                    uint8_t *stg = tiles + OUT_STAGING_OFFSET + epi_warp * OUT_STAGING_WARP_BYTES;
+                    // The unit's last tile has the rings to itself (its MMAs are done, no load
+                    // follows): all four boxes are staged side by side and leave together.
+                    // Otherwise a warp's boxes go through its own buffer (two of them in the one-CTA
+                    // form, which has half the epilogue warps), each after the one before it in that
+                    // buffer has been read.
+                    const bool last = seg == n_seg - 1;
+                    constexpr int OWN = CG == 1 ? 2 : 1;
+                    uint8_t *base = last ? tiles + epi_warp * (4 * OUT_STAGING_WARP_BYTES)
+                                         : tiles + OUT_STAGING_OFFSET + epi_warp * (OWN * OUT_STAGING_WARP_BYTES);
                     const int row_base = row - lane;
 #pragma unroll
                     for (int ch = 0; ch < 4; ++ch) {
-                        // the previous box must have been read out of the staging buffer
-                        if (lane == 0) bulk_wait_read_all();
-                        __syncwarp();
+                        uint8_t *stg = base + (last ? ch : ch % OWN) * OUT_STAGING_WARP_BYTES;
+                        if (!last) {
+                            if (lane == 0) bulk_wait_read<OWN - 1>();
+                            __syncwarp();
+                        }
 #pragma unroll
                         for (int c = 0; c < 8; ++c)
                             *reinterpret_cast<float4 *>(stg + lane * 128 + ((c ^ (lane & 7)) << 4)) =
@@ -1257,6 +1275,33 @@ __global__ void __launch_bounds__(Cfg<CG>::NUM_THREADS, 1) gemm_f32_3xtf32_kerne
                         }
                         __syncwarp();
                     }
+                } else if (args.c_sj == 1) {
+                    // Rows of C that start anywhere: the same staging, stored 32 adjacent words at a
+                    // time (a thread storing its own row makes every instruction touch 32 lines).
+                    uint8_t *stg = tiles + OUT_STAGING_OFFSET + epi_warp * OUT_STAGING_WARP_BYTES;
+                    const int row_base = row - lane;
+                    float *cbase = args.c + static_cast<long long>(b) * args.c_sb;
+#pragma unroll
+                    for (int ch = 0; ch < 4; ++ch) {
+#pragma unroll
+                        for (int c = 0; c < 8; ++c)
+                            *reinterpret_cast<float4 *>(stg + lane * 128 + ((c ^ (lane & 7)) << 4)) =
+                                make_float4(sum[ch * 32 + 4 * c], sum[ch * 32 + 4 * c + 1], sum[ch * 32 + 4 * c + 2],
+                                            sum[ch * 32 + 4 * c + 3]);
+                        __syncwarp();
+                        const int gcol = col0 + ch * 32 + lane;
+                        if (gcol < args.M) {
+                            float *dst = cbase + static_cast<long long>(row_base) * args.c_si + gcol;
+#pragma unroll 8
+                            for (int r = 0; r < 32; ++r) {
+                                const float v =
+                                    *reinterpret_cast<const float *>(stg + r * 128 + (((lane >> 2) ^ (r & 7)) << 4) + (lane & 3) * 4);
+                                if (row_base + r < args.N) *dst = v;
+                                dst += args.c_si;
+                            }
+                        }
+                        __syncwarp();
+                    }
                 } else if (mine) {
 #pragma unroll
                     for (int j = 0; j < 128; ++j)
@@ -1281,9 +1326,12 @@ __global__ void __launch_bounds__(Cfg<CG>::NUM_THREADS, 1) gemm_f32_3xtf32_kerne
         // Bulk tensor stores still in flight read this CTA's shared memory: they must be done
         // before the CTA gives it up.
         if (lane == 0) {
-            bulk_wait_all();
+            bulk_wait_read<0>();
             // stores to peer GPUs must have left this GPU before the kernel is reported complete
-            if (args.n_peers > 0 || args.mc_c != nullptr) __threadfence_system();
+            if (args.n_peers > 0 || args.mc_c != nullptr) {
+                bulk_wait_all();
+                __threadfence_system();
+            }
         }
         if (args.prof && warp == C::FIRST_EPI_WARP && lane == 0) {
             if (PROF) args.prof[blockIdx.x * kProfSlots + kProfEpiAccFull] = w_a;

@@ -410,7 +410,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_i32_limb_kernel(const __g
                     const int row_base = row - lane;
 #pragma unroll
                     for (int ch = 0; ch < 2; ++ch) {
-                        if (lane == 0) bulk_wait_read_all();  // the previous box has left the buffer
+                        if (lane == 0) bulk_wait_read<0>();  // the previous box has left the buffer
                         __syncwarp();
 #pragma unroll
                         for (int c = 0; c < 8; ++c)
@@ -442,7 +442,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_i32_limb_kernel(const __g
             acc_phase ^= 1u;
         }
         // Bulk tensor stores in flight read this CTA's shared memory: done before it is given up.
-        if (lane == 0) bulk_wait_all();
+        if (lane == 0) bulk_wait_read<0>();
     } else if (warp >= FIRST_CONV_WARP) {
         // ------------------------------------------------------------ converters
         const int r = threadIdx.x - FIRST_CONV_WARP * 32;  // 0..127: the row of A this thread splits

@@ -1,18 +1,16 @@
 // gemm_skinny.cuh -- bandwidth-bound products with one tiny dim (included by gemm_simt.cu).
 //
-// A classifier head or its gradient (tinytensor's MNIST example: H[4096,1024] . W2^T[1024,10],
-// dC[4096,10] . W2[10,1024], H^T[1024,4096] . dC[4096,10]) has 5-20 flops per byte: what counts
-// is reading the large operand once, coalesced, with the tiny one kept on chip.  The register-
-// tiled kernel spends its time on tile bookkeeping there (16-22 us for 17 MB); these three
-// kernels stream:
-//   row_dot      M <= 16, lhs rows contiguous along K: a warp per output row, lanes walk K,
-//                rhs transposed in shared memory, M warp-reduced sums per row;
-//   col_stream   M <= 16, lhs contiguous along its rows (a transposed view): a thread per
-//                output row, the K range of the CTA's split streamed with the rhs slice
-//                broadcast from shared memory; partial sums per split, fixed-order reduce;
-//   outer        K <= 16: a thread per four output columns, lhs row and rhs rows from L1.
+// A vector times a weight matrix, a classifier head or its gradients (tinytensor's MNIST example:
+// H[4096,1024] . W2[1024,10], dC[4096,10] . W2^T[10,1024], H^T[1024,4096] . dC[4096,10]) has 0.5-20
+// flops per byte: what counts is reading (or writing) the large operand once, in wide accesses
+// with enough of them in flight (about 44 KB per SM at 6.5 TB/s), the tiny one kept on chip.
+//   row_dot      M <= 16, lhs rows contiguous along K: a warp per output row, lanes walk K, the rhs
+//                transposed in shared memory;
+//   col_stream   M <= 16, lhs contiguous along its rows (a transposed view; a row-major weight
+//                matrix under a vector): lanes walk the rows, warps and CTAs of a cluster split K;
+//   outer        K <= 16: a thread keeps its columns of rhs in registers and walks rows of C.
 // All dtypes; integer sums wrap as everywhere else (unsigned accumulators); the fused addend /
-// relu is applied by whoever writes the final value.
+// relu is applied by whoever writes the final value.  No scratch memory, one launch each.
 #pragma once
 
 namespace skinny {
@@ -24,6 +22,43 @@ template <typename T>
 struct alignas(sizeof(T) * 4 > 16 ? 16 : sizeof(T) * 4) Vec4T {
     T v[4];
 };
+
+__device__ __forceinline__ uint32_t cluster_rank() {
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// The object at `p` (this CTA's shared memory) as seen in CTA `rank` of the cluster.
+template <typename A>
+__device__ __forceinline__ const A *in_cta(const A *p, uint32_t rank) {
+    uint64_t out;
+    asm volatile("mapa.u64 %0, %1, %2;" : "=l"(out) : "l"(reinterpret_cast<uint64_t>(p)), "r"(rank));
+    return reinterpret_cast<const A *>(out);
+}
+
+// put(i, get(i)) for i in [0, COUNT) by 256 threads, eight loads in flight before the first store (left
+// to itself the compiler waits for each).
+template <int COUNT, typename Get, typename Put>
+__device__ __forceinline__ void stage(Get get, Put put) {
+    constexpr int STEPS = (COUNT + 255) / 256, BATCH = STEPS < 8 ? STEPS : 8;
+#pragma unroll 1
+    for (int s = 0; s < STEPS; s += BATCH) {
+        decltype(get(0)) v[BATCH];
+#pragma unroll
+        for (int u = 0; u < BATCH; ++u) {
+            const int idx = threadIdx.x + (s + u) * 256;
+            if (idx < COUNT) v[u] = get(idx);
+        }
+#pragma unroll
+        for (int u = 0; u < BATCH; ++u) {
+            const int idx = threadIdx.x + (s + u) * 256;
+            if (idx < COUNT) put(idx, v[u]);
+        }
+    }
+}
 
 // ---- row_dot: out[b,n,j] = sum_k A[b,n,k] B[b,k,j], a_sk == 1.  MC = m_cols rounded up to 4.
 // grid (CTAs striding over rows, B); block 1024 = 32 warps, a warp per row at a time; dynamic
@@ -80,95 +115,192 @@ __global__ void __launch_bounds__(1024) row_dot_kernel(SimtArgs p, int m_cols) {
     }
 }
 
-// ---- col_stream: out[b,i,j] (+)= sum over this split's k of A[b,i,k] B[b,k,j], a_si == 1.
-// grid (row blocks of 128, splits, B); block 128.  With splits > 1 the destination is the split's
-// slab of the scratch ([split][B][N][M], contiguous) and the epilogue is left to the reduce.
-template <typename T, int MC>
-__global__ void __launch_bounds__(128) col_stream_kernel(SimtArgs p, int m_cols) {
+// ---- col_stream: out[b,i,j] = sum_k A[b,i,k] B[b,k,j], a_si == 1.  MC >= m_cols.
+// LX lanes side by side take four rows i each, the other 256 / LX threads of a column and the
+// CTAs of a cluster (grid.y) split K; 8 four-element loads in flight per thread.  The sums meet
+// in shared memory and then across the cluster (distributed shared memory), always in the
+// same order.  VEC: the i's of a lane are adjacent and start on a four-element boundary.
+// Vector [4096] . W[4096,4096]: 121.5 us (a thread per row, 4 loads in flight, and a second
+// kernel for the reduction) -> 12.6 us = 5.3 TB/s.
+template <typename T, int MC, int LX, bool VEC>
+__global__ void __launch_bounds__(256) col_stream_kernel(SimtArgs p, int m_cols) {
     using A = typename AccOf<T>::type;
-    constexpr int KC = 128;  // rhs rows staged at a time
+    constexpr int RY = 256 / LX;                                  // threads along K
+    constexpr int COLS = LX * 4;                                  // rows i of this CTA
+    // rhs rows staged at a time: with few columns a CTA, enough for eight loads by each of the 256 / LX threads
+    constexpr int KC = (MC == 1 ? 512 : (sizeof(A) == 8 ? 1024 : 2048) * (LX < 32 ? 3 : 1) / MC) & ~(RY - 1);
+    constexpr int U = sizeof(T) == 8 ? 4 : 8;
+    constexpr int JG = MC < 4 ? MC : (sizeof(A) == 8 ? 2 : 4);    // columns j reduced at a time
     __shared__ __align__(16) A bs[KC][MC];
+    __shared__ A red[8][JG][COLS];
+    __shared__ A part[MC][COLS];
+    const int warp = threadIdx.x >> 5;
+    const int lx = threadIdx.x % LX, ky = threadIdx.x / LX;
     const long long batch = blockIdx.z;
-    const int split = blockIdx.y;
-    const long long k_begin = static_cast<long long>(split) * p.k_per_split;
+    const long long k_begin = static_cast<long long>(blockIdx.y) * p.k_per_split;
     const long long k_end = (k_begin + p.k_per_split < p.K) ? k_begin + p.k_per_split : p.K;
-    const T *__restrict__ a = static_cast<const T *>(p.a) + batch * p.a_sb;
     const T *__restrict__ b = static_cast<const T *>(p.b) + batch * p.b_sb;
-    T *__restrict__ c = static_cast<T *>(p.c) + batch * p.c_sb + static_cast<long long>(split) * p.c_ss;
-    const long long i = static_cast<long long>(blockIdx.x) * 128 + threadIdx.x;
-    A acc[MC];
+    T *__restrict__ c = static_cast<T *>(p.c) + batch * p.c_sb;
+    const long long i0 = static_cast<long long>(blockIdx.x) * COLS;
+    const long long i = VEC ? i0 + lx * 4 : i0 + lx;
+    constexpr int ISTEP = VEC ? 1 : LX;
+    const T *__restrict__ a = static_cast<const T *>(p.a) + batch * p.a_sb + i;
+    const bool whole = VEC && i + 4 <= p.N;
+    A acc[MC][4];
 #pragma unroll
-    for (int j = 0; j < MC; ++j) acc[j] = A(0);
+    for (int j = 0; j < MC; ++j)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) acc[j][e] = A(0);
     for (long long k0 = k_begin; k0 < k_end; k0 += KC) {
         const int kc = static_cast<int>(k_end - k0 < KC ? k_end - k0 : KC);
+        if (k0 > k_begin) __syncthreads();
+        stage<KC * MC>(
+            [&](int idx) {
+                const int kk = idx / MC, j = idx % MC;
+                return kk < kc && j < m_cols ? widen<T>(b[(k0 + kk) * p.b_sk + j * p.b_sj]) : A(0);
+            },
+            [&](int idx, A v) { bs[idx / MC][idx % MC] = v; });
         __syncthreads();
-        for (int idx = threadIdx.x; idx < kc * MC; idx += 128) {
-            const int kk = idx / MC, j = idx % MC;  // columns past m_cols are zero: no predicate below
-            bs[kk][j] = j < m_cols ? widen<T>(b[(k0 + kk) * p.b_sk + j * p.b_sj]) : A(0);
-        }
-        __syncthreads();
-        if (i < p.N) {
-            const T *__restrict__ col = a + i + k0 * p.a_sk;
-#pragma unroll 4
-            for (int kk = 0; kk < kc; ++kk) {
-                const A av = widen<T>(col[kk * p.a_sk]);
+        const T *__restrict__ col = a + k0 * p.a_sk;
+        for (int kb = ky; kb < kc; kb += RY * U) {
+            Vec4T<T> v[U];
 #pragma unroll
-                for (int j4 = 0; j4 < MC; j4 += 4) {
-                    const Vec4T<A> bv = *reinterpret_cast<const Vec4T<A> *>(&bs[kk][j4]);  // broadcast read
-#pragma unroll
-                    for (int u = 0; u < 4; ++u) acc[j4 + u] = mad<A>(av, bv.v[u], acc[j4 + u]);
-                }
-            }
-        }
-    }
-    if (i < p.N) {
-#pragma unroll
-        for (int j = 0; j < MC; ++j)
-            if (j < m_cols) c[i * p.c_si + j * p.c_sj] = finish<T>(acc[j], p.ep, batch, i, j);
-    }
-}
-
-// ---- outer: out[b,n,j..j+3] = sum_{k < K <= 16} A[b,n,k] B[b,k,j..j+3].  One thread per four
-// columns; grid (rows, column-group blocks, B) so that no index needs a division.
-template <typename T>
-__global__ void __launch_bounds__(256) outer_kernel(SimtArgs p, int k_dim, int b_vec, int c_vec) {
-    using A = typename AccOf<T>::type;
-    const long long n = blockIdx.x, batch = blockIdx.z;
-    const long long g = static_cast<long long>(blockIdx.y) * 256 + threadIdx.x;
-    if (g * 4 >= p.M) return;
-    {
-        const T *__restrict__ a = static_cast<const T *>(p.a) + batch * p.a_sb + n * p.a_si;
-        const T *__restrict__ b = static_cast<const T *>(p.b) + batch * p.b_sb;
-        T *__restrict__ c = static_cast<T *>(p.c) + batch * p.c_sb + n * p.c_si;
-        const bool full = g * 4 + 4 <= p.M;
-        A acc[4] = {A(0), A(0), A(0), A(0)};
-#pragma unroll
-        for (int k = 0; k < kMaxSmall; ++k) {
-            if (k < k_dim) {
-                const A av = widen<T>(a[k * p.a_sk]);
-                if (b_vec && full) {
-                    const Vec4T<T> bv = *reinterpret_cast<const Vec4T<T> *>(b + k * p.b_sk + g * 4);
-#pragma unroll
-                    for (int u = 0; u < 4; ++u) acc[u] = mad<A>(av, widen<T>(bv.v[u]), acc[u]);
+            for (int u = 0; u < U; ++u) {
+                const int kk = kb + u * RY;
+                if (whole && kk < kc) {
+                    v[u] = *reinterpret_cast<const Vec4T<T> *>(col + kk * p.a_sk);
                 } else {
 #pragma unroll
-                    for (int u = 0; u < 4; ++u) {
-                        const long long j = g * 4 + u;
-                        if (j < p.M) acc[u] = mad<A>(av, widen<T>(b[k * p.b_sk + j * p.b_sj]), acc[u]);
-                    }
+                    for (int e = 0; e < 4; ++e)
+                        v[u].v[e] = kk < kc && i + e * ISTEP < p.N ? col[kk * p.a_sk + e * ISTEP] : T(0);
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const int kk = kb + u * RY;
+                if (kk >= kc) break;
+#pragma unroll
+                for (int j = 0; j < MC; ++j) {
+                    const A bv = bs[kk][j];
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) acc[j][e] = mad<A>(widen<T>(v[u].v[e]), bv, acc[j][e]);
                 }
             }
         }
-        if (c_vec && full) {
+    }
+    // lanes of a warp that share a column
+    if constexpr (LX < 32) {
+#pragma unroll
+        for (int off = 16; off >= LX; off >>= 1)
+#pragma unroll
+            for (int j = 0; j < MC; ++j)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) acc[j][e] = acc[j][e] + __shfl_xor_sync(0xFFFFFFFFu, acc[j][e], off);
+    }
+    // the eight warps
+#pragma unroll
+    for (int j0 = 0; j0 < MC; j0 += JG) {
+        __syncthreads();
+        if ((threadIdx.x & 31) < LX) {
+#pragma unroll
+            for (int j = 0; j < JG; ++j)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) red[warp][j][VEC ? lx * 4 + e : lx + e * LX] = acc[j0 + j][e];
+        }
+        __syncthreads();
+        for (int idx = threadIdx.x; idx < JG * COLS; idx += 256) {
+            A s = A(0);
+#pragma unroll
+            for (int w = 0; w < 8; ++w) s = s + red[w][idx / COLS][idx % COLS];
+            part[j0 + idx / COLS][idx % COLS] = s;
+        }
+    }
+    // the CTAs of the cluster: CTA r finishes every gridDim.y-th element
+    const uint32_t splits = gridDim.y;
+    uint32_t rank = 0;
+    if (splits > 1) {
+        cluster_sync();
+        rank = cluster_rank();
+    } else {
+        __syncthreads();
+    }
+    for (int idx = static_cast<int>(rank) * 256 + threadIdx.x; idx < m_cols * COLS; idx += static_cast<int>(splits) * 256) {
+        const int j = idx / COLS, ii = idx % COLS;
+        if (i0 + ii >= p.N) continue;
+        A s = A(0);
+        if (splits > 1) {
+            for (uint32_t r = 0; r < splits; ++r) s = s + *in_cta(&part[j][ii], r);
+        } else {
+            s = part[j][ii];
+        }
+        c[(i0 + ii) * p.c_si + j * p.c_sj] = finish<T>(s, p.ep, batch, i0 + ii, j);
+    }
+    if (splits > 1) cluster_sync();  // nobody leaves while its sums are being read
+}
+
+// ---- outer: out[b,n,j] = sum_{k < K <= KT} A[b,n,k] B[b,k,j].
+// 64 x 4 threads take 256 columns x ROWS rows: a thread keeps its four columns of rhs (K x 4
+// values) in registers and walks ROWS / 4 rows, whose lhs values come from shared memory.  Bound by
+// the writes of C.  (One thread per row and four columns read rhs again for every row:
+// 4096 x 10 x 1024 took 51.9 us, now 5.9.)
+// VEC: rows of C start on a four-element boundary.  grid (row blocks, column blocks, B).
+template <typename T, int KT, int ROWS, bool VEC>
+__global__ void __launch_bounds__(256) outer_kernel(SimtArgs p) {
+    using A = typename AccOf<T>::type;
+    __shared__ __align__(16) A as[ROWS][KT];
+    __shared__ __align__(16) A bs[KT][256 + 16 / sizeof(A)];
+    const int tx = threadIdx.x & 63, ty = threadIdx.x >> 6;
+    const long long batch = blockIdx.z;
+    const long long n0 = static_cast<long long>(blockIdx.x) * ROWS, j0 = static_cast<long long>(blockIdx.y) * 256;
+    const T *__restrict__ a = static_cast<const T *>(p.a) + batch * p.a_sb;
+    const T *__restrict__ b = static_cast<const T *>(p.b) + batch * p.b_sb;
+    T *__restrict__ c = static_cast<T *>(p.c) + batch * p.c_sb;
+    const int K = static_cast<int>(p.K);
+    const bool ka_fast = p.a_sk <= p.a_si;
+    stage<ROWS * KT>(
+        [&](int idx) {
+            const int r = ka_fast ? idx / KT : idx % ROWS, k = ka_fast ? idx % KT : idx / ROWS;
+            return k < K && n0 + r < p.N ? widen<T>(a[(n0 + r) * p.a_si + k * p.a_sk]) : A(0);
+        },
+        [&](int idx, A v) { as[ka_fast ? idx / KT : idx % ROWS][ka_fast ? idx % KT : idx / ROWS] = v; });
+    // (through shared memory: the rhs is often a transposed view, whose columns lie K apart)
+    const bool kb_fast = p.b_sk < p.b_sj;
+    stage<256 * KT>(
+        [&](int idx) {
+            const int jj = kb_fast ? idx / KT : idx % 256, k = kb_fast ? idx % KT : idx / 256;
+            return k < K && j0 + jj < p.M ? widen<T>(b[k * p.b_sk + (j0 + jj) * p.b_sj]) : A(0);
+        },
+        [&](int idx, A v) { bs[kb_fast ? idx % KT : idx / 256][kb_fast ? idx / KT : idx % 256] = v; });
+    const long long j = VEC ? j0 + tx * 4 : j0 + tx;
+    constexpr int JSTEP = VEC ? 1 : 64;
+    A bv[KT][4];
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < KT; ++k)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) bv[k][e] = bs[k][VEC ? tx * 4 + e : tx + e * 64];
+#pragma unroll 2
+    for (int r = ty; r < ROWS; r += 4) {
+        const long long n = n0 + r;
+        if (n >= p.N) break;
+        A acc[4] = {A(0), A(0), A(0), A(0)};
+#pragma unroll
+        for (int k = 0; k < KT; ++k) {
+            const A av = as[r][k];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) acc[e] = mad<A>(av, bv[k][e], acc[e]);
+        }
+        T *crow = c + n * p.c_si;
+        if (VEC && j + 4 <= p.M) {
             Vec4T<T> out;
 #pragma unroll
-            for (int u = 0; u < 4; ++u) out.v[u] = finish<T>(acc[u], p.ep, batch, n, g * 4 + u);
-            *reinterpret_cast<Vec4T<T> *>(c + g * 4) = out;
+            for (int e = 0; e < 4; ++e) out.v[e] = finish<T>(acc[e], p.ep, batch, n, j + e);
+            *reinterpret_cast<Vec4T<T> *>(crow + j) = out;
         } else {
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                const long long j = g * 4 + u;
-                if (j < p.M) c[j * p.c_sj] = finish<T>(acc[u], p.ep, batch, n, j);
+            for (int e = 0; e < 4; ++e) {
+                const long long je = j + e * JSTEP;
+                if (je < p.M) crow[je * p.c_sj] = finish<T>(acc[e], p.ep, batch, n, je);
             }
         }
     }

@@ -1,0 +1,113 @@
+// pack_f32.cu -- f32 operands whose rows TMA cannot describe (a base or a pitch that is not a
+// multiple of 16 bytes: 769 columns, a view that starts at column 1) copied into padded rows, so that
+// a product large enough for the tcgen05 kernel gets it.  The copy moves each operand once; the
+// product reads it N / 256 or M / 256 times.
+//
+// A warp takes a row, 32 adjacent words per instruction, eight in flight.  Both operands go in
+// one launch.  1003 x 769 and 769 x 1251: 4.4 us, and the product then takes 25 us where the
+// CUDA-core kernel took 121.
+#include "common.cuh"
+
+namespace ttb {
+
+int workspace_slot(int device, cudaStream_t stream, int slot, size_t bytes, void **out);
+
+namespace {
+
+constexpr int kPackSlot = 4;  // workspace slots 4 (lhs) and 5 (rhs)
+
+struct PackOne {
+    const float *src;
+    float *dst;
+    long long rows, inner, row_stride, batch_stride, pitch;  // elements
+    long long total_rows;                                    // rows * batches; 0 = nothing to copy
+};
+
+__global__ void __launch_bounds__(256) pack_rows_kernel(PackOne a, PackOne b) {
+    const int lane = threadIdx.x & 31;
+    const long long warp0 = static_cast<long long>(blockIdx.x) * 8 + (threadIdx.x >> 5);
+    for (long long w = warp0; w < a.total_rows + b.total_rows; w += static_cast<long long>(gridDim.x) * 8) {
+        const bool second = w >= a.total_rows;
+        const PackOne &o = second ? b : a;
+        const long long r = second ? w - a.total_rows : w;
+        const float *src = o.src + (r / o.rows) * o.batch_stride + (r % o.rows) * o.row_stride;
+        float *dst = o.dst + r * o.pitch;
+        for (long long i0 = lane; i0 < o.inner; i0 += 256) {
+            float v[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u)
+                if (i0 + u * 32 < o.inner) v[u] = src[i0 + u * 32];
+#pragma unroll
+            for (int u = 0; u < 8; ++u)
+                if (i0 + u * 32 < o.inner) dst[i0 + u * 32] = v[u];
+        }
+    }
+}
+
+// Rows [batch][row] of `inner` adjacent elements, in padded form.
+struct Rows {
+    const void *src;
+    long long rows, inner, row_stride, batch_stride, batches;
+};
+
+bool aligned(const Rows &o) {
+    return (reinterpret_cast<uintptr_t>(o.src) & 15) == 0 && (o.rows == 1 || (o.row_stride > 0 && (o.row_stride & 3) == 0)) &&
+           (o.batches == 1 || (o.batch_stride & 3) == 0);
+}
+
+int prepare(const Problem &p, const Rows &o, int slot, PackOne *one, void **dst) {
+    if (aligned(o)) return TTB_OK;
+    one->pitch = (o.inner + 3) / 4 * 4;
+    const long long batches = o.batch_stride == 0 ? 1 : o.batches;
+    int rc = workspace_slot(p.device, p.stream, slot, static_cast<size_t>(batches) * o.rows * one->pitch * 4, dst);
+    if (rc != TTB_OK) return rc;
+    one->src = static_cast<const float *>(o.src);
+    one->dst = static_cast<float *>(*dst);
+    one->rows = o.rows;
+    one->inner = o.inner;
+    one->row_stride = o.row_stride;
+    one->batch_stride = o.batch_stride;
+    one->total_rows = batches * o.rows;
+    return TTB_OK;
+}
+
+}  // namespace
+
+// `p` with operands that TMA can describe.  Needs unit stride along one matrix dim of each operand.
+// Fails (and leaves `p` as it was) when no workspace can be had.
+int pack_f32_operands(Problem *p) {
+    const bool a_k = p->a_sk == 1 || p->K == 1, b_k = p->b_sk == 1 || p->K == 1;
+    const Rows a = a_k ? Rows{p->a, p->N, p->K, p->a_si, p->a_sb, p->B} : Rows{p->a, p->K, p->N, p->a_sk, p->a_sb, p->B};
+    const Rows b = b_k ? Rows{p->b, p->M, p->K, p->b_sj, p->b_sb, p->B} : Rows{p->b, p->K, p->M, p->b_sk, p->b_sb, p->B};
+    PackOne pa{}, pb{};
+    pa.rows = pb.rows = 1;
+    void *da = nullptr, *db = nullptr;
+    int rc = prepare(*p, a, kPackSlot, &pa, &da);
+    if (rc == TTB_OK) rc = prepare(*p, b, kPackSlot + 1, &pb, &db);
+    if (rc != TTB_OK) return rc;
+    const long long rows = pa.total_rows + pb.total_rows;
+    if (rows == 0) return TTB_OK;
+    int sms = 148;
+    sm_count(p->device, &sms);
+    long long blocks = (rows + 7) / 8;
+    if (blocks > 8LL * sms) blocks = 8LL * sms;
+    pack_rows_kernel<<<static_cast<unsigned>(blocks), 256, 0, p->stream>>>(pa, pb);
+    cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return cuda_fail(e, "pack_rows_kernel launch");
+    note_launch(-1, 1);
+    if (da != nullptr) {
+        p->a = da;
+        p->a_si = a_k ? pa.pitch : 1;
+        p->a_sk = a_k ? 1 : pa.pitch;
+        p->a_sb = a.batch_stride == 0 ? 0 : pa.pitch * a.rows;
+    }
+    if (db != nullptr) {
+        p->b = db;
+        p->b_sj = b_k ? pb.pitch : 1;
+        p->b_sk = b_k ? 1 : pb.pitch;
+        p->b_sb = b.batch_stride == 0 ? 0 : pb.pitch * b.rows;
+    }
+    return TTB_OK;
+}
+
+}  // namespace ttb

@@ -43,13 +43,15 @@ struct Options {
     int a_tmem = 0;              // f32 hybrid split: correction MMAs read their A operands from tensor memory
     int extra_conv = 1;          // f32 pair form: warps 2-3 convert 5/8 of every B tile
     int sk_pair = -1;            // f32 tensor-core kernel: paired stream-K (-1 automatic, 0 never, 1 whenever possible)
+    int mma_tile = -1;           // mma.sync f32 kernel, forced: tile and K splits (see launch_f32_mma)
+    int mma_splits = 0;
     int pieces = -1;             // f32 tensor-core kernel: piece schedule (-1 automatic, 0 never, n parts per tile)
 };
 Options g_opt;
 
 constexpr int kMaxDevices = 64;
 constexpr int kMaxStreamKSets = 8;
-constexpr int kExtraSlots = 3;
+constexpr int kExtraSlots = 5;
 constexpr int kHostChunks = 8;  // pipeline depth of the host-buffer entry point
 struct StreamKSet {
     cudaStream_t stream;
@@ -222,7 +224,7 @@ int streamk_workspace(int device, cudaStream_t stream, float **partials, unsigne
 // Cached scratch buffers, one per (device, stream, slot), grown on demand.  Slot 0: split-K
 // partial sums of the CUDA-core kernels; 1: conv2d's unrolled columns; 2: conv2d's
 // weight-gradient partials; 3: conv2d's padded weights (the products conv2d runs may use slot 0
-// at the same time, hence separate slots).  Keyed by stream so that calls on different streams
+// at the same time, hence separate slots); 4 and 5: f32 operands copied into padded rows.  Keyed by stream so that calls on different streams
 // of one device never share partial sums; calls on ONE stream are ordered by the stream.
 // Growing replaces the buffer: cudaFree synchronises the device, so kernels that still use the
 // old one have finished -- except launches recorded into a CUDA graph, which run again later.
@@ -435,6 +437,62 @@ int resolve_problem(const ttb_view *lhs, const ttb_view *rhs, void *out, int dty
 static int dispatch(const Problem &p);
 int dispatch_problem(const Problem &p) { return dispatch(p); }
 
+// CTA pairs (256 x 256 tiles) halve shared-memory and L2 traffic per flop; they pay off once the output
+// is more than one 128-wide tile in both dims and there are enough pair tiles to occupy a good part
+// of the GPU.  Fewer pair tiles are fine when K is long: stream-K then deals the K blocks out over
+// all pairs (16 or more each).
+static int launch_f32_tc(const Problem &p, int sms) {
+    const long long pair_tiles = ((p.N + 255) / 256) * ((p.M + 255) / 256) * p.B;
+    const long long kb = (p.K + 31) / 32;
+    const bool enough = pair_tiles >= 24 || (g_opt.streamk != 0 && kb >= 64 && pair_tiles * kb / (sms / 2) >= 16);
+    const bool pair = g_opt.two_cta < 0 ? (p.N > 128 && p.M > 128 && enough) : g_opt.two_cta != 0;
+    return launch_f32_tcgen05(p, f32_options(pair));
+}
+
+static int launch_mma_as(const Problem &p, int variant) {
+    const int rc = launch_f32_mma(p);
+    if (rc == TTB_OK) note_launch(variant, 1);
+    return rc;
+}
+
+// Automatic dispatch of an f32 product.
+static int dispatch_f32(const Problem &p, int sms) {
+    char why[160] = "";
+    const bool mma = f32_mma_eligible(p);
+    if (p.N <= 16 || p.M <= 16 || p.K <= 16) {
+        // Streaming products.  With 2 to 16 columns (or rows) under a K of 64 or more the tensor core
+        // takes the multiply-adds off the cores that have to keep the loads going (4096 x 1024 x 10:
+        // 15.9 -> 8.5 us); a lone vector, or a tiny K, is all loads or stores anyway.
+        const bool flip = p.N < p.M;
+        const int64_t tiny = flip ? p.N : p.M, other = flip ? p.M : p.N;
+        if (mma && tiny >= 2 && other >= 32 && p.K >= 64) {
+            const Problem q = flip ? transposed(p) : p;
+            if (f32_mma_eligible(q)) return launch_mma_as(q, TTB_VARIANT_SIMT_SKINNY);
+        }
+        if (p.K <= 16 || other < 32 || tiny == 1 || !mma) return launch_simt(p, g_opt.splitk != 0, true);
+        return launch_mma_as(p, TTB_VARIANT_MMA_F32);
+    }
+    const double work = static_cast<double>(p.N) * p.M * p.K * p.B;
+    const bool tma = f32_tcgen05_eligible(p, why, sizeof(why));
+    // The tcgen05 kernel starts from about 8 us and then is five times as fast as mma.sync.  A single
+    // product crosses over between 2^28 and 2^29 multiply-adds (512^3 = 2^27: 9.7-10.6 against 19.1 us;
+    // 1024^3 = 2^30: 47 against 29); a batched one, whose tiles fill the SMs at a smaller K, sooner
+    // (256 x 128 x 64 x 128 = 2^28: 17.5 against 12.2).  Operands that have to be copied first move
+    // the line by the copy, some 5 us, and so do products that fill less than half of a 128-wide
+    // tile (64 x 32 x 25 x 576: 4.4 against 14.9).
+    const bool sliver = p.N < 64 || p.M < 64;
+    const double line = !tma || sliver ? 536870912.0 : p.B == 1 ? 268435456.0 : 8388608.0;
+    if (mma && work < line) return launch_mma_as(p, TTB_VARIANT_MMA_F32);
+    if (tma) return launch_f32_tc(p, sms);
+    if (mma) {
+        Problem q = p;
+        if (pack_f32_operands(&q) == TTB_OK && f32_tcgen05_eligible(q, why, sizeof(why))) return launch_f32_tc(q, sms);
+        set_error("%s", "");  // no workspace (a stream capture, say): the kernel that needs none
+        return launch_mma_as(p, TTB_VARIANT_MMA_F32);
+    }
+    return launch_simt(p, g_opt.splitk != 0, true);
+}
+
 static int dispatch(const Problem &p) {
     DeviceState *d;
     int rc = device_state(p.device, &d);
@@ -465,6 +523,15 @@ static int dispatch(const Problem &p) {
                 return TTB_EUNSUPPORTED;
             }
             return launch_f64_dmma(p);
+        case TTB_VARIANT_MMA_F32: {
+            if (!f32_mma_eligible(p)) {
+                set_error("forced mma.sync f32 variant cannot take this call");
+                return TTB_EUNSUPPORTED;
+            }
+            rc = launch_f32_mma(p, g_opt.mma_tile, g_opt.mma_splits);
+            if (rc == TTB_OK) note_launch(TTB_VARIANT_MMA_F32, 1);
+            return rc;
+        }
         case TTB_VARIANT_TCGEN05_I8LIMB:
             if (!i32_tcgen05_eligible(p, why, sizeof(why))) {
                 set_error("forced int8-plane tcgen05 variant cannot take this call: %s", why);
@@ -474,25 +541,7 @@ static int dispatch(const Problem &p) {
         default: break;
     }
     // Automatic dispatch.
-    if (p.dtype == TTB_F32) {
-        // Tensor cores pay off once the product has enough work per output tile;
-        // skinny outputs (a dim <= 16) are bandwidth-bound and go to the SIMT kernel.
-        const bool big = p.N > 16 && p.M > 16 && p.K >= 16 &&
-                         static_cast<double>(p.N) * p.M * p.K * p.B >= 128.0 * 128.0 * 64.0;
-        if (big && f32_tcgen05_eligible(p, why, sizeof(why))) {
-            // CTA pairs (256x256 tiles) halve shared-memory and L2 traffic per flop; they
-            // pay off once the output is more than one 128-wide tile in both dims and there
-            // are enough pair tiles to occupy a good part of the GPU.
-            // Fewer pair tiles are fine when K is long: stream-K then deals the K blocks out over
-            // all pairs (16 or more each).
-            const long long pair_tiles = ((p.N + 255) / 256) * ((p.M + 255) / 256) * p.B;
-            const long long kb = (p.K + 31) / 32;
-            const bool enough = pair_tiles >= 24 || (g_opt.streamk != 0 && kb >= 64 && pair_tiles * kb / (d->sms / 2) >= 16);
-            const bool pair = g_opt.two_cta < 0 ? (p.N > 128 && p.M > 128 && enough) : g_opt.two_cta != 0;
-            return launch_f32_tcgen05(p, f32_options(pair));
-        }
-        return launch_simt(p, g_opt.splitk != 0, true);
-    }
+    if (p.dtype == TTB_F32) return dispatch_f32(p, d->sms);
     if (p.dtype == TTB_F64) {
         if (p.N > 16 && p.M > 16 && p.K > 16 && f64_dmma_eligible(p)) return launch_f64_dmma(p);
         return launch_simt(p, g_opt.splitk != 0, true);
@@ -840,6 +889,7 @@ TTB_API const char *ttb_variant_name(int variant) {
         case TTB_VARIANT_TCGEN05_2CTA: return "tcgen05_3xtf32_2cta";
         case TTB_VARIANT_TCGEN05_I8LIMB: return "tcgen05_i8_byte_planes";
         case TTB_VARIANT_SIMT_SKINNY: return "simt_skinny";
+        case TTB_VARIANT_MMA_F32: return "mma_f32";
         default: return "unknown";
     }
 }
@@ -850,7 +900,7 @@ TTB_API int ttb_set_option(const char *key, int64_t value) {
         return TTB_EINVAL;
     }
     if (!strcmp(key, "force_variant")) {
-        if (value < 0 || value > TTB_VARIANT_TCGEN05_I8LIMB) {
+        if (value < 0 || value > TTB_VARIANT_MMA_F32 || value == TTB_VARIANT_SIMT_SKINNY) {
             set_error("force_variant: %lld is not a variant", static_cast<long long>(value));
             return TTB_EINVAL;
         }
@@ -929,6 +979,22 @@ TTB_API int ttb_set_option(const char *key, int64_t value) {
         g_opt.pieces = static_cast<int>(value);
         return TTB_OK;
     }
+    if (!strcmp(key, "mma_tile")) {
+        if (value < -1 || value > 4) {
+            set_error("mma_tile must be -1 (by shape) or 0..4");
+            return TTB_EINVAL;
+        }
+        g_opt.mma_tile = static_cast<int>(value);
+        return TTB_OK;
+    }
+    if (!strcmp(key, "mma_splits")) {
+        if (value != 0 && value != 1 && value != 2 && value != 4 && value != 8) {
+            set_error("mma_splits must be 0 (by shape), 1, 2, 4 or 8");
+            return TTB_EINVAL;
+        }
+        g_opt.mma_splits = static_cast<int>(value);
+        return TTB_OK;
+    }
     if (!strcmp(key, "extra_conv")) {
         g_opt.extra_conv = value != 0;
         return TTB_OK;
@@ -965,6 +1031,8 @@ TTB_API int64_t ttb_get_option(const char *key) {
     if (!strcmp(key, "a_tmem")) return g_opt.a_tmem;
     if (!strcmp(key, "extra_conv")) return g_opt.extra_conv;
     if (!strcmp(key, "pieces")) return g_opt.pieces;
+    if (!strcmp(key, "mma_tile")) return g_opt.mma_tile;
+    if (!strcmp(key, "mma_splits")) return g_opt.mma_splits;
     if (!strcmp(key, "sk_pair")) return g_opt.sk_pair;
     set_error("unknown option '%s'", key);
     return TTB_EINVAL;
