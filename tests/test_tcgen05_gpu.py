@@ -388,3 +388,16 @@ def test_profile_counters_do_not_change_results(forced, level):
         busy = prof[:, 5]
         assert busy.max() > 0 and np.all(busy <= total.max())
     forced.check_device(0)
+
+
+@pytest.mark.parametrize("M", [576, 520, 132])
+def test_boxes_outside_c_between_tiles_of_one_unit(forced, M):
+    """Several tiles per CTA, the last column of tiles only partly inside C: the boxes that are not
+    stored must not let a later one overwrite a staging buffer that is still being read."""
+    rng = np.random.default_rng(47)
+    a = rng.standard_normal((1, 128, 64)).astype(np.float32)
+    b = rng.standard_normal((160, 64, M)).astype(np.float32)
+    A, Bm = dev(a).expand(160, 128, 64), dev(b)
+    want = np.matmul(a.astype(np.float64), b.astype(np.float64))
+    for _ in range(3):
+        assert rel_to_max(host(forced.batched_matmul(A, Bm)), want) <= F32_TOL

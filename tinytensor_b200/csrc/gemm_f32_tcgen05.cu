@@ -1236,8 +1236,10 @@ __global__ void __launch_bounds__(Cfg<CG>::NUM_THREADS, 1) gemm_f32_3xtf32_kerne
                             // peer GPU's C over NVLink, straight from the staging buffer.
                             for (int pr = 0; pr < args.n_peers; ++pr)
                                 tma_store_3d(&args.tmap_peer[pr], stg, gcol, row_base, b * args.c_batch_mul);
-                            bulk_commit_group();
                         }
+                        // One group per box, an empty one for a box outside C: the wait above counts
+                        // groups to tell which of the two buffers has been read.
+                        if (lane == 0) bulk_commit_group();
                     }
                 } else if (vec_ok) {
                     // Same staging, stored by the warp itself (fused all-gather: the forwarding
