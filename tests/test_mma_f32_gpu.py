@@ -1,7 +1,7 @@
 """The mma.sync f32 kernel and the padded copy in front of the tcgen05 kernel, at the edges: every
 tile and K split, both layouts of both operands, remainders in every dim, rows that start anywhere,
 Inf / NaN, and fused epilogues with a C whose rows are unaligned.  Gate: 1e-5 of the largest
-result, as for every f32 kernel (the split leaves 2^-19 per product)."""
+result, as for every f32 kernel; and against 64 bits no further off than fp32 multiply-adds."""
 import numpy as np
 import pytest
 import torch
@@ -119,3 +119,36 @@ def test_padded_copy_is_not_needed_in_a_capture(ttb):
     torch.cuda.synchronize()
     assert rel_to_max(host(out), np.matmul(a.astype(np.float64), b.astype(np.float64))) <= F32_TOL
     ttb.check_device(0)
+
+
+@pytest.mark.parametrize("shape", [(1, 33, 20, 31), (1, 200, 17, 200), (1, 128, 64, 96), (1, 512, 512, 512), (1, 500, 333, 201),
+                                   (1, 64, 2048, 64), (1, 2000, 1024, 10), (1, 1003, 769, 1251), (1, 1031, 385, 1403)])
+def test_no_less_exact_than_fp32(ttb, shape):
+    """Rounding each of K additions to 24 bits leaves 2^-24 / sqrt(12) of a partial sum, which grows as
+    sqrt(k): 2^-24 sqrt(K / 24) of the result.  A bound of twice that, at least 2^-22.5 (three TF32
+    products leave 2^-23 to 2^-22 whatever K is)."""
+    rng = np.random.default_rng(106)
+    B, N, K, M = shape
+    a, A = _operand(rng, (B, N, K), False, 1)
+    b, Bm = _operand(rng, (B, K, M), False, 0)
+    want = np.matmul(a.astype(np.float64), b.astype(np.float64))
+    err = np.linalg.norm(host(ttb.batched_matmul(A, Bm)) - want) / np.linalg.norm(want)
+    assert err <= max(2.0 ** -23 * (K / 24) ** 0.5, 2.0 ** -22.5)
+
+
+@pytest.mark.parametrize("low,high", [(-126, -100), (-149, -120), (100, 126)])
+def test_words_at_the_ends_of_the_range(options, low, high):
+    """Words whose last bits lie below bf16's smallest number are multiplied as fp32 words, next to
+    ordinary ones and alone; results that are denormal themselves are off by a bit of 2^-149."""
+    rng = np.random.default_rng(107)
+    options.set_option("force_variant", int(options.Variant.MMA_F32))
+    N, K, M = 45, 70, 37
+    a = np.ldexp(rng.uniform(1, 2, (1, N, K)), rng.integers(low, high, (1, N, K))).astype(np.float32)
+    b = (rng.standard_normal((1, K, M)) * (2.0 ** -8 if high > 0 else 1)).astype(np.float32)
+    b[0, 0::7] = 0
+    for x in (a, np.where(rng.random((1, N, K)) < 0.5, a, rng.standard_normal((1, N, K)).astype(np.float32))):
+        want = np.matmul(x.astype(np.float64), b.astype(np.float64))
+        size = np.matmul(np.abs(x).astype(np.float64), np.abs(b).astype(np.float64))
+        got = host(options.batched_matmul(dev(x), dev(b)))
+        # K products of at most `size` in all, each addition rounded
+        assert (np.abs(got - want) <= K * (2.0 ** -24 * size + 2.0 ** -149)).all()

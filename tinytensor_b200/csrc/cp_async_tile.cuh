@@ -1,0 +1,102 @@
+// cp_async_tile.cuh -- operand tiles brought into shared memory by cp.async, for kernels that run
+// on warp-level tensor-core instructions (gemm_f32_mma.cu), and the cluster
+// helpers with which they add up sums over a K split.
+#pragma once
+
+#include <cstdint>
+
+namespace ttb {
+
+__device__ __forceinline__ uint32_t smem_addr(const void *p) {
+    return static_cast<uint32_t>(__cvta_generic_to_shared(p));
+}
+// bytes < 16 (or < 8, < 4): the rest of the destination is zero-filled.
+__device__ __forceinline__ void cp16(uint32_t dst, const void *src, int bytes) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+}
+template <int SIZE>
+__device__ __forceinline__ void cp_one(uint32_t dst, const void *src, int bytes) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %3, %2;" ::"r"(dst), "l"(src), "r"(bytes), "n"(SIZE) : "memory");
+}
+__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_wait() {
+    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+__device__ __forceinline__ uint32_t cluster_rank() {
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+template <typename E>
+__device__ __forceinline__ const E *in_cta(const E *p, uint32_t rank) {
+    uint64_t out;
+    asm volatile("mapa.u64 %0, %1, %2;" : "=l"(out) : "l"(reinterpret_cast<uint64_t>(p)), "r"(rank));
+    return reinterpret_cast<const E *>(out);
+}
+
+// Brings BK-deep slices of an operand tile of ROWS rows (A) or columns (B) into shared memory:
+// [row][k] with a pitch of BK + 4 words, or, for an operand contiguous along its rows (MN),
+// [k][row] with a pitch of ROWS + 32 bytes: both make the fragment reads conflict-free.  A thread's
+// pieces lie `step` apart in memory and a constant apart in shared memory, in K (MN) or along the
+// rows, so that a piece costs an addition, a comparison and the copy: 16 bytes (`vec`: the view is
+// aligned) or one word of any view.
+template <typename E, int BK, int ROWS, bool MN, int THREADS>
+struct TileLoader {
+    static constexpr int SIZE = sizeof(E), WIDE = 16 / SIZE;
+    static constexpr int PITCH = MN ? ROWS + 32 / SIZE : BK + 4;
+    static constexpr int WORDS = PITCH * (MN ? BK : ROWS);
+    const E *p;            // this thread's first piece of the next slice
+    long long step;        // elements from piece to piece
+    long long slice_step;  // elements from slice to slice
+    uint32_t dst;          // byte offset of the first piece in the slice
+    int left;              // rows left from this thread's first one (not MN), or of them loaded by a piece (MN)
+    int k;                 // first k of this thread within a slice
+    bool vec;
+
+    __device__ TileLoader(const E *src, long long s_row, long long s_k, int row0, int rows, int k0, bool vec_) : vec(vec_) {
+        const int wide = vec ? WIDE : 1;
+        const int across = (MN ? ROWS : BK) / wide;  // pieces side by side
+        const int x = static_cast<int>(threadIdx.x) % across * wide, y = static_cast<int>(threadIdx.x) / across;
+        const int r = MN ? x : y;
+        k = MN ? y : x;
+        p = src + (row0 + r) * s_row + (k0 + k) * s_k;
+        step = (THREADS / across) * (MN ? s_k : s_row);
+        slice_step = BK * s_k;
+        dst = static_cast<uint32_t>((MN ? k * PITCH + r : r * PITCH + k) * SIZE);
+        left = rows - row0 - r;
+    }
+    // The next slice, of which k_left k's exist.
+    __device__ __forceinline__ void load(uint32_t slice, int k_left) {
+        k_left -= k;
+        const uint32_t to = slice + dst;
+        constexpr int N = MN ? BK : ROWS;
+        const int words = MN ? left : k_left;  // along a piece
+        const int lines = MN ? k_left : left;
+        const E *from = p;
+        if (vec) {
+            constexpr int ACROSS = (MN ? ROWS : BK) / WIDE, DOWN = THREADS / ACROSS;
+            const int bytes = words >= WIDE ? 16 : (words > 0 ? words * SIZE : 0);
+#pragma unroll
+            for (int i = 0; i < (N + DOWN - 1) / DOWN; ++i) {
+                if (N % DOWN != 0 && static_cast<int>(threadIdx.x) / ACROSS + i * DOWN >= N) break;
+                cp16(to + i * DOWN * PITCH * SIZE, from, i * DOWN < lines ? bytes : 0);
+                from += step;
+            }
+        } else {
+            constexpr int ACROSS = MN ? ROWS : BK, DOWN = THREADS / ACROSS;
+            static_assert(N % DOWN == 0, "one word per thread and line");
+#pragma unroll
+            for (int i = 0; i < N / DOWN; ++i) {
+                cp_one<SIZE>(to + i * DOWN * PITCH * SIZE, from, words > 0 && i * DOWN < lines ? SIZE : 0);
+                from += step;
+            }
+        }
+        p += slice_step;
+    }
+};
+
+}  // namespace ttb

@@ -11,34 +11,34 @@
 // cluster split K when the tiles alone would leave SMs idle (sums meet through distributed
 // shared memory: one launch, no scratch, fixed order).
 //
-// Arithmetic: the hybrid split of the tcgen05 kernel (see gemm_f32_tcgen05.cu): x = big + small with
-// big = x truncated to TF32, A.B = big.big (TF32) + bf16(small_A).bf16(B) + bf16(A).bf16(small_B).  An
-// m16n8k16 bf16 fragment holds two k's per register where two m16n8k8 TF32 fragments hold k and
-// k + 4; any pairing of k's is right as long as A and B agree, so the bf16 fragments are packed from
-// the TF32 ones in place.  Non-finite elements are zero in the bf16 operands and travel through
-// the TF32 product alone.  The tensor core's accumulator does not round to nearest, so every 256
-// of K it is added into fp32 registers and restarted.
+// Arithmetic: as exact as fp32 multiply-adds, because that is what these products are otherwise
+// given (a small or unaligned product, one of few columns).  A word is the sum of three bf16 numbers
+// (8 bits each, cut off, exact); six of the nine products are formed, smallest first, and what
+// is left out is under 2^-24 of a product.  Each 16 of K the tensor core's sum, which is not rounded
+// to nearest, is added into fp32 registers: 1.1e-7 off in the 2-norm at K = 64 and 2.3e-7 at 2047,
+// fp32 multiply-adds in sequence 1.4e-7 and 8.1e-7.  (TF32 products with bf16 corrections, the
+// tcgen05 kernel's split, take the same time here and are 1.3e-6 off.)  An m16n8k16 bf16 fragment
+// holds two k's per register; any pairing of k's is right as long as A and B agree, so the fragments
+// are packed from words k and k + 4, which is how ldmatrix deals them.
 //
-// Bounds: two TF32 and two bf16 instructions per 16 x 8 x 16, at the measured 275 and 550 TFLOP/s of
-// mma.sync, give 137 TFLOP/s; a large product reaches 62 (tensor pipe 45 % active: with 160 registers
-// a scheduler holds three warps, too few to hide the chain of reads, splits and MMAs), so large ones
-// go to the tcgen05 kernel.  Small ones, device time against that kernel and the CUDA-core one:
-// 32 x 128 x 512 9.7 -> 4.1 us, 512^3 19.7 -> 9.7-10.6, 64 x 2048 x 64 36.6 -> 7.4,
-// 500 x 333 x 201 25.0 -> 7.3, 4096 x 1024 x 10 15.9 -> 8.5.
+// Bounds: six bf16 instructions per 16 x 8 x 16, at the measured 550 TFLOP/s of mma.sync, give 92
+// TFLOP/s; a large product reaches 41 (2047^3; with 168 registers a scheduler holds three warps,
+// too few to hide the chain of reads, cuts and MMAs), so large ones go to the tcgen05 kernel.
+// Small ones, device time against that kernel and the CUDA-core one: 32 x 128 x 512 9.7 -> 4.1 us,
+// 512^3 19.7 -> 10.6, 64 x 2048 x 64 36.6 -> 7.4, 500 x 333 x 201 25.0 -> 7.3,
+// 4096 x 1024 x 10 15.9 -> 8.5.
 //
 // Replaces matmul_kernel<float> of the reference for these sizes and views
 // (tinytensor/tensor/backend/cuda/kernel/matmul.cuh:27-151).
-#include <cuda_bf16.h>
-
 #include <atomic>
 
 #include "common.cuh"
+#include "cp_async_tile.cuh"
 
 namespace ttb {
 namespace {
 
 constexpr int BK = 32;
-constexpr int FOLD_KB = 8;  // K blocks between additions of the tensor core's sums into registers
 
 struct MmaArgs {
     const float *a;
@@ -54,67 +54,38 @@ struct MmaArgs {
     Epilogue ep;
 };
 
-__device__ __forceinline__ uint32_t smem_addr(const void *p) {
-    return static_cast<uint32_t>(__cvta_generic_to_shared(p));
-}
-// bytes < 16 (or < 4): the rest of the destination is zero-filled.
-__device__ __forceinline__ void cp16(uint32_t dst, const void *src, int bytes) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void cp4(uint32_t dst, const void *src, int bytes) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_wait() {
-    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
-}
-__device__ __forceinline__ uint32_t cluster_rank() {
-    uint32_t r;
-    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-    return r;
-}
-__device__ __forceinline__ void cluster_sync() {
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-__device__ __forceinline__ const float *in_cta(const float *p, uint32_t rank) {
-    uint64_t out;
-    asm volatile("mapa.u64 %0, %1, %2;" : "=l"(out) : "l"(reinterpret_cast<uint64_t>(p)), "r"(rank));
-    return reinterpret_cast<const float *>(out);
-}
-
-__device__ __forceinline__ void mma_tf32(float (&c)[4], const uint32_t (&a)[4], const uint32_t (&b)[2]) {
-    asm volatile(
-        "mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
-        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
-}
 __device__ __forceinline__ void mma_bf16(float (&c)[4], const uint32_t (&a)[4], const uint32_t (&b)[2]) {
     asm volatile(
         "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
         : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
         : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
 }
-
-// Two fp32 words of one fragment position (k and k + 4): their TF32 parts, and bf16 pairs of the low
-// parts and of the values themselves.  `z` stays finite as long as every word seen is finite: the
-// low part of Inf and NaN is NaN, and NaN survives every multiply-add after it.
-__device__ __forceinline__ void split2(float x, float y, uint32_t &bx, uint32_t &by, uint32_t &s, uint32_t &v, float &z) {
-    bx = __float_as_uint(x) & 0xFFFFE000u;
-    by = __float_as_uint(y) & 0xFFFFE000u;
-    const float dx = x - __uint_as_float(bx), dy = y - __uint_as_float(by);
-    const __nv_bfloat162 p = __floats2bfloat162_rn(dx, dy);
-    const __nv_bfloat162 q = __floats2bfloat162_rn(x, y);
-    z = fmaf(dx, dy, z);
-    s = *reinterpret_cast<const uint32_t *>(&p);
-    v = *reinterpret_cast<const uint32_t *>(&q);
+// c = a . b
+__device__ __forceinline__ void mma_bf16_first(float (&c)[4], const uint32_t (&a)[4], const uint32_t (&b)[2]) {
+    asm volatile(
+        "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%10, %10, %10, %10};"
+        : "=f"(c[0]), "=f"(c[1]), "=f"(c[2]), "=f"(c[3])
+        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]), "f"(0.0f));
 }
-// Zeroes the bf16 entries whose low part is NaN, that is, those of Inf and NaN.
-__device__ __forceinline__ void keep_finite(uint32_t &s, uint32_t &v) {
-    const __nv_bfloat162 p = *reinterpret_cast<const __nv_bfloat162 *>(&s);
-    const uint32_t keep = __heq2_mask(p, p);
-    s &= keep;
-    v &= keep;
+
+// Two fp32 words of one fragment position (k and k + 4), each cut into three bf16 numbers of 8 bits whose
+// sum is the word.  Words for which that cannot be (Inf, NaN, and those below 2^-109, whose last
+// bits are under bf16's smallest denormal) leave a remainder with bits below a bf16's: `rest` collects them.
+struct Cut {
+    uint32_t h, m, l;
+};
+__device__ __forceinline__ Cut cut2(uint32_t x, uint32_t y, uint32_t &rest) {
+    Cut c;
+    c.h = __byte_perm(x, y, 0x7632);
+    const float rx = __uint_as_float(x) - __uint_as_float(x & 0xFFFF0000u);
+    const float ry = __uint_as_float(y) - __uint_as_float(y & 0xFFFF0000u);
+    const uint32_t ux = __float_as_uint(rx), uy = __float_as_uint(ry);
+    c.m = __byte_perm(ux, uy, 0x7632);
+    const uint32_t lx = __float_as_uint(rx - __uint_as_float(ux & 0xFFFF0000u));
+    const uint32_t ly = __float_as_uint(ry - __uint_as_float(uy & 0xFFFF0000u));
+    c.l = __byte_perm(lx, ly, 0x7632);
+    rest |= lx | ly;
+    return c;
 }
 // Four 8 x 4 blocks of fp32 words, one word per thread of each: row (lane / 4), word (lane % 4) of the
 // block whose row r starts at the address lane 8 * block + r passes.
@@ -125,64 +96,8 @@ __device__ __forceinline__ void ldmatrix4(uint32_t (&v)[4], uint32_t addr) {
                  : "memory");
 }
 
-// Brings BK-deep slices of an operand tile of ROWS rows (A) or columns (B) into shared memory:
-// [row][k] with a pitch of BK + 4 words, or, for an operand contiguous along its rows (MN),
-// [k][row] with a pitch of ROWS + 8: both make the fragment reads conflict-free.  A thread's
-// pieces lie `step` apart in memory and a constant apart in shared memory, in K (MN) or along the
-// rows, so that a piece costs an addition, a comparison and the copy.
 template <int ROWS, bool MN, int THREADS>
-struct Loader {
-    static constexpr int PITCH = MN ? ROWS + 8 : BK + 4;
-    const float *p;        // this thread's first piece of the next slice
-    long long step;        // elements from piece to piece
-    long long slice_step;  // elements from slice to slice
-    uint32_t dst;          // byte offset of the first piece in the slice
-    int left;              // rows left from this thread's first one (not MN), or of them loaded by a piece (MN)
-    int k;                 // first k of this thread within a slice
-    bool vec;
-
-    __device__ Loader(const float *src, long long s_row, long long s_k, int row0, int rows, int k0, bool vec_) : vec(vec_) {
-        const int wide = vec ? 4 : 1;
-        const int across = (MN ? ROWS : BK) / wide;  // pieces side by side
-        const int x = static_cast<int>(threadIdx.x) % across * wide, y = static_cast<int>(threadIdx.x) / across;
-        const int r = MN ? x : y;
-        k = MN ? y : x;
-        p = src + (row0 + r) * s_row + (k0 + k) * s_k;
-        step = (THREADS / across) * (MN ? s_k : s_row);
-        slice_step = BK * s_k;
-        dst = static_cast<uint32_t>((MN ? k * PITCH + r : r * PITCH + k) * 4);
-        left = rows - row0 - r;
-    }
-    // The next slice, of which k_left k's exist.
-    __device__ __forceinline__ void load(uint32_t slice, int k_left) {
-        k_left -= k;
-        const uint32_t to = slice + dst;
-        if (vec) {
-            constexpr int ACROSS = (MN ? ROWS : BK) / 4, DOWN = THREADS / ACROSS, N = (MN ? BK : ROWS);
-            const int words = MN ? left : k_left;  // of the 4 of a piece
-            const int bytes = words >= 4 ? 16 : (words > 0 ? words * 4 : 0);
-            const int lines = MN ? k_left : left;
-            const float *from = p;
-#pragma unroll
-            for (int i = 0; i < (N + DOWN - 1) / DOWN; ++i) {
-                if (N % DOWN != 0 && static_cast<int>(threadIdx.x) / ACROSS + i * DOWN >= N) break;
-                cp16(to + i * DOWN * PITCH * 4, from, i * DOWN < lines ? bytes : 0);
-                from += step;
-            }
-        } else {
-            constexpr int ACROSS = MN ? ROWS : BK, DOWN = THREADS / ACROSS, N = (MN ? BK : ROWS);
-            const bool in = (MN ? left : k_left) > 0;
-            const int lines = MN ? k_left : left;
-            const float *from = p;
-#pragma unroll
-            for (int i = 0; i < N / DOWN; ++i) {
-                cp4(to + i * DOWN * PITCH * 4, from, in && i * DOWN < lines ? 4 : 0);
-                from += step;
-            }
-        }
-        p += slice_step;
-    }
-};
+using Loader = TileLoader<float, BK, ROWS, MN, THREADS>;
 
 __device__ __forceinline__ float finish(float v, const Epilogue &ep, long long b, int i, int j) {
     if (ep.d) v += static_cast<const float *>(ep.d)[b * ep.d_sb + i * ep.d_si + j * ep.d_sj];
@@ -232,13 +147,13 @@ __global__ void __launch_bounds__(WARPS_M *WARPS_N *WARPS_K * 32, MIN_CTAS) gemm
         k_left -= BK;
     };
 
-    float acc[MI][NI][4], sum[MI][NI][4];
+    float sum[MI][NI][4];
 #pragma unroll
     for (int i = 0; i < MI; ++i)
 #pragma unroll
         for (int j = 0; j < NI; ++j)
 #pragma unroll
-            for (int r = 0; r < 4; ++r) acc[i][j][r] = sum[i][j][r] = 0.0f;
+            for (int r = 0; r < 4; ++r) sum[i][j][r] = 0.0f;
 
     const int num_kb = k_end > k_begin ? (k_end - k_begin + BK - 1) / BK : 0;
 #pragma unroll
@@ -258,9 +173,7 @@ __global__ void __launch_bounds__(WARPS_M *WARPS_N *WARPS_K * 32, MIN_CTAS) gemm
 #pragma unroll
         for (int k1 = 0; k1 < BK / WARPS_K; k1 += 16) {
             const int k = WARPS_K == 2 ? wk * 16 : k1;
-            uint32_t a_big[MI][2][4], a_low[MI][4], a_val[MI][4];
-            uint32_t b_big[NI][2][2], b_low[NI][2], b_val[NI][2];
-            float z = 0.0f;
+            uint32_t ah[MI][4], am[MI][4], al[MI][4], bh[NI][2], bm[NI][2], bl[NI][2], rest = 0;
 #pragma unroll
             for (int j = 0; j < NI; ++j) {
                 // words (k + t, k + t + 4, k + 8 + t, k + 12 + t) of column g
@@ -273,9 +186,12 @@ __global__ void __launch_bounds__(WARPS_M *WARPS_N *WARPS_K * 32, MIN_CTAS) gemm
                     ldmatrix4(w, bs32 + ((wn + j * 8 + (lane & 7)) * PB + k + (lane >> 3) * 4) * 4);
                 }
 #pragma unroll
-                for (int h = 0; h < 2; ++h)
-                    split2(__uint_as_float(w[2 * h]), __uint_as_float(w[2 * h + 1]), b_big[j][h][0], b_big[j][h][1],
-                           b_low[j][h], b_val[j][h], z);
+                for (int h = 0; h < 2; ++h) {
+                    const Cut c = cut2(w[2 * h], w[2 * h + 1], rest);
+                    bh[j][h] = c.h;
+                    bm[j][h] = c.m;
+                    bl[j][h] = c.l;
+                }
             }
 #pragma unroll
             for (int i = 0; i < MI; ++i)
@@ -291,55 +207,65 @@ __global__ void __launch_bounds__(WARPS_M *WARPS_N *WARPS_K * 32, MIN_CTAS) gemm
                         ldmatrix4(w, as32 + ((wm + i * 16 + u * 8 + (lane & 7)) * PA + k + (lane >> 3) * 4) * 4);
                     }
 #pragma unroll
-                    for (int h = 0; h < 2; ++h)
-                        split2(__uint_as_float(w[2 * h]), __uint_as_float(w[2 * h + 1]), a_big[i][h][u], a_big[i][h][u + 2],
-                               a_low[i][h * 2 + u], a_val[i][h * 2 + u], z);
-                }
-            if (!(fabsf(z) <= 3.0e38f)) {
-#pragma unroll
-                for (int j = 0; j < NI; ++j)
-#pragma unroll
-                    for (int h = 0; h < 2; ++h) keep_finite(b_low[j][h], b_val[j][h]);
-#pragma unroll
-                for (int i = 0; i < MI; ++i)
-#pragma unroll
-                    for (int q = 0; q < 4; ++q) keep_finite(a_low[i][q], a_val[i][q]);
-            }
-            __syncwarp();
-            // (one kind at a time over all tiles: a tile's next instruction comes MI x NI later)
-#pragma unroll
-            for (int i = 0; i < MI; ++i)
-#pragma unroll
-                for (int j = 0; j < NI; ++j) mma_bf16(acc[i][j], a_low[i], b_val[j]);
-#pragma unroll
-            for (int i = 0; i < MI; ++i)
-#pragma unroll
-                for (int j = 0; j < NI; ++j) mma_bf16(acc[i][j], a_val[i], b_low[j]);
-#pragma unroll
-            for (int h = 0; h < 2; ++h)
-#pragma unroll
-                for (int i = 0; i < MI; ++i)
-#pragma unroll
-                    for (int j = 0; j < NI; ++j) mma_tf32(acc[i][j], a_big[i][h], b_big[j][h]);
-        }
-        if ((kb & (FOLD_KB - 1)) == FOLD_KB - 1) {
-#pragma unroll
-            for (int i = 0; i < MI; ++i)
-#pragma unroll
-                for (int j = 0; j < NI; ++j)
-#pragma unroll
-                    for (int r = 0; r < 4; ++r) {
-                        sum[i][j][r] += acc[i][j][r];
-                        acc[i][j][r] = 0.0f;
+                    for (int h = 0; h < 2; ++h) {
+                        const Cut c = cut2(w[2 * h], w[2 * h + 1], rest);
+                        ah[i][h * 2 + u] = c.h;
+                        am[i][h * 2 + u] = c.m;
+                        al[i][h * 2 + u] = c.l;
                     }
+                }
+            if (__any_sync(0xFFFFFFFFu, (rest & 0xFFFFu) != 0)) {
+                // a word that cannot be cut: these 16 k's by multiply-adds of the words themselves
+#pragma unroll 1
+                for (int q = k; q < k + 16; ++q) {
+                    float y[NI][2];
+#pragma unroll
+                    for (int j = 0; j < NI; ++j)
+#pragma unroll
+                        for (int e = 0; e < 2; ++e) {
+                            const int col = wn + j * 8 + 2 * t + e;
+                            y[j][e] = bs[B_MN ? q * PB + col : col * PB + q];
+                        }
+#pragma unroll
+                    for (int i = 0; i < MI; ++i)
+#pragma unroll
+                        for (int u = 0; u < 2; ++u) {
+                            const int row = wm + i * 16 + g + 8 * u;
+                            const float x = as[A_MN ? q * PA + row : row * PA + q];
+#pragma unroll
+                            for (int j = 0; j < NI; ++j)
+#pragma unroll
+                                for (int e = 0; e < 2; ++e) sum[i][j][2 * u + e] = fmaf(x, y[j][e], sum[i][j][2 * u + e]);
+                        }
+                }
+                continue;
+            }
+            // (one kind at a time over all tiles: a tile's next instruction comes MI x NI later; smallest
+            // first, so that only the last of the six is cut at the size of the whole)
+            float acc[MI][NI][4];
+            auto products = [&](const uint32_t(&x)[MI][4], const uint32_t(&y)[NI][2]) {
+#pragma unroll
+                for (int i = 0; i < MI; ++i)
+#pragma unroll
+                    for (int j = 0; j < NI; ++j) mma_bf16(acc[i][j], x[i], y[j]);
+            };
+#pragma unroll
+            for (int i = 0; i < MI; ++i)
+#pragma unroll
+                for (int j = 0; j < NI; ++j) mma_bf16_first(acc[i][j], al[i], bh[j]);
+            products(ah, bl);
+            products(am, bm);
+            products(am, bh);
+            products(ah, bm);
+            products(ah, bh);
+#pragma unroll
+            for (int i = 0; i < MI; ++i)
+#pragma unroll
+                for (int j = 0; j < NI; ++j)
+#pragma unroll
+                    for (int r = 0; r < 4; ++r) sum[i][j][r] += acc[i][j][r];
         }
     }
-#pragma unroll
-    for (int i = 0; i < MI; ++i)
-#pragma unroll
-        for (int j = 0; j < NI; ++j)
-#pragma unroll
-            for (int r = 0; r < 4; ++r) sum[i][j][r] += acc[i][j][r];
 
     constexpr int PS = BN + 4;
     auto leave_sums = [&]() {

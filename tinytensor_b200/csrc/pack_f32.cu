@@ -4,7 +4,7 @@
 // product reads it N / 256 or M / 256 times.
 //
 // A warp takes a row, 32 adjacent words per instruction, eight in flight.  Both operands go in
-// one launch.  1003 x 769 and 769 x 1251: 4.4 us, and the product then takes 25 us where the
+// one launch.  1003 x 769 and 769 x 1251: 4.4 us, and the product then takes 31 us where the
 // CUDA-core kernel took 121.
 #include "common.cuh"
 
@@ -15,6 +15,7 @@ int workspace_slot(int device, cudaStream_t stream, int slot, size_t bytes, void
 namespace {
 
 constexpr int kPackSlot = 4;  // workspace slots 4 (lhs) and 5 (rhs)
+constexpr size_t kPackMost = size_t(1) << 30;  // bytes of a copy; the workspace is kept for the stream's next call
 
 struct PackOne {
     const float *src;
@@ -59,7 +60,9 @@ int prepare(const Problem &p, const Rows &o, int slot, PackOne *one, void **dst)
     if (aligned(o)) return TTB_OK;
     one->pitch = (o.inner + 3) / 4 * 4;
     const long long batches = o.batch_stride == 0 ? 1 : o.batches;
-    int rc = workspace_slot(p.device, p.stream, slot, static_cast<size_t>(batches) * o.rows * one->pitch * 4, dst);
+    const size_t bytes = static_cast<size_t>(batches) * o.rows * one->pitch * 4;
+    if (bytes > kPackMost) return TTB_ELIMIT;
+    int rc = workspace_slot(p.device, p.stream, slot, bytes, dst);
     if (rc != TTB_OK) return rc;
     one->src = static_cast<const float *>(o.src);
     one->dst = static_cast<float *>(*dst);
@@ -74,7 +77,8 @@ int prepare(const Problem &p, const Rows &o, int slot, PackOne *one, void **dst)
 }  // namespace
 
 // `p` with operands that TMA can describe.  Needs unit stride along one matrix dim of each operand.
-// Fails (and leaves `p` as it was) when no workspace can be had.
+// Fails (and leaves `p` as it was) when no workspace can be had
+// or a copy would be larger than the limit.
 int pack_f32_operands(Problem *p) {
     const bool a_k = p->a_sk == 1 || p->K == 1, b_k = p->b_sk == 1 || p->K == 1;
     const Rows a = a_k ? Rows{p->a, p->N, p->K, p->a_si, p->a_sb, p->B} : Rows{p->a, p->K, p->N, p->a_sk, p->a_sb, p->B};

@@ -441,12 +441,17 @@ int dispatch_problem(const Problem &p) { return dispatch(p); }
 // is more than one 128-wide tile in both dims and there are enough pair tiles to occupy a good part
 // of the GPU.  Fewer pair tiles are fine when K is long: stream-K then deals the K blocks out over
 // all pairs (16 or more each).
-static int launch_f32_tc(const Problem &p, int sms) {
+static int launch_f32_tc(const Problem &p, int sms, bool full_split = false) {
     const long long pair_tiles = ((p.N + 255) / 256) * ((p.M + 255) / 256) * p.B;
     const long long kb = (p.K + 31) / 32;
     const bool enough = pair_tiles >= 24 || (g_opt.streamk != 0 && kb >= 64 && pair_tiles * kb / (sms / 2) >= 16);
     const bool pair = g_opt.two_cta < 0 ? (p.N > 128 && p.M > 128 && enough) : g_opt.two_cta != 0;
-    return launch_f32_tcgen05(p, f32_options(pair));
+    F32Options o = f32_options(pair);
+    if (full_split) {
+        o.terms = 3;
+        o.k_chunk = 1;
+    }
+    return launch_f32_tcgen05(p, o);
 }
 
 static int launch_mma_as(const Problem &p, int variant) {
@@ -485,8 +490,14 @@ static int dispatch_f32(const Problem &p, int sms) {
     if (mma && work < line) return launch_mma_as(p, TTB_VARIANT_MMA_F32);
     if (tma) return launch_f32_tc(p, sms);
     if (mma) {
+        // Views that TMA cannot describe are multiplied in fp32 or as exactly.  Copied into padded rows
+        // they take three TF32 products and an fp32 addition every K block: 3.5e-7 off at any K, where
+        // an fp32 sum is 1.8e-8 sqrt(K) off, so from K = 384; 1003 x 769 x 1251 51 us, mma.sync 76,
+        // CUDA cores 119.  (The bf16 corrections of aligned views: 45 us, but 2.0e-6 off.)  Below,
+        // mma.sync is 1.3e-7 off: 2047 x 301 x 1999 84 us, CUDA cores 96.
         Problem q = p;
-        if (pack_f32_operands(&q) == TTB_OK && f32_tcgen05_eligible(q, why, sizeof(why))) return launch_f32_tc(q, sms);
+        if (p.K >= 384 && pack_f32_operands(&q) == TTB_OK && f32_tcgen05_eligible(q, why, sizeof(why)))
+            return launch_f32_tc(q, sms, true);
         set_error("%s", "");  // no workspace (a stream capture, say): the kernel that needs none
         return launch_mma_as(p, TTB_VARIANT_MMA_F32);
     }
