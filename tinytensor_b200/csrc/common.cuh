@@ -107,7 +107,8 @@ int pack_f32_operands(Problem *p);
 // two_cta: -1 = pick CTA pairs by shape, 0 = never, 1 = always.
 int launch_i32_tcgen05(const Problem &p, int two_cta = -1, int dbg = 0);
 bool i32_tcgen05_eligible(const Problem &p, char *why, int why_len);
-int launch_f64_dmma(const Problem &p);
+// tile: -1 = by shape, else 0 (64 x 64), 1 (32 x 32); splits of K over a cluster: 0 = by shape.
+int launch_f64_dmma(const Problem &p, int tile = -1, int splits = 0);
 int measure_fp64_tensor_peak(int device, double *tflops);
 bool f64_dmma_eligible(const Problem &p);
 

@@ -1,5 +1,5 @@
-// cp_async_tile.cuh -- operand tiles brought into shared memory by cp.async, for kernels that run
-// on warp-level tensor-core instructions (gemm_f32_mma.cu), and the cluster
+// cp_async_tile.cuh -- operand tiles brought into shared memory by cp.async, for the kernels that run
+// on warp-level tensor-core instructions (gemm_f32_mma.cu, gemm_f64_dmma.cu), and the cluster
 // helpers with which they add up sums over a K split.
 #pragma once
 

@@ -533,7 +533,7 @@ static int dispatch(const Problem &p) {
                 set_error("forced DMMA variant cannot take this call");
                 return TTB_EUNSUPPORTED;
             }
-            return launch_f64_dmma(p);
+            return launch_f64_dmma(p, g_opt.mma_tile, g_opt.mma_splits);
         case TTB_VARIANT_MMA_F32: {
             if (!f32_mma_eligible(p)) {
                 set_error("forced mma.sync f32 variant cannot take this call");
