@@ -383,7 +383,9 @@ __device__ __forceinline__ void forward_tile(const TcArgs &args, int t, int cta_
 
 // PROF: the roles count the cycles they wait and work (ttb_tc_profile); the clock reads cost each
 // role a few dozen cycles per K block, so the counting build is a kernel of its own.
-template <int CG, bool PROF>
+// RAGGED: rows of C that TMA cannot describe (in a kernel of its own: the code of that store in the
+// other one's epilogue, never run, slowed 8192^3 by 3.5 %).
+template <int CG, bool PROF, bool RAGGED>
 __global__ void __launch_bounds__(Cfg<CG>::NUM_THREADS, 1) gemm_f32_3xtf32_kernel(const __grid_constant__ TcArgs args) {
     using C = Cfg<CG>;
     constexpr bool PAIR = CG == 2;
@@ -913,8 +915,10 @@ __global__ void __launch_bounds__(Cfg<CG>::NUM_THREADS, 1) gemm_f32_3xtf32_kerne
                 tc_fence_after_sync();
                 const uint32_t t_row = tmem_base + static_cast<uint32_t>(acc * C::ACC_COLS + col_half * 128) +
                                        (static_cast<uint32_t>(quarter * 32) << 16);
-                if (ch == kb0) {
+                const bool first = ch == kb0;
+                if (CG == 1 && first) {
                     // the first chunk of a tile is the sum so far: one wait for all 128 columns
+                    // (tiles of few chunks, which the one-CTA form is given, wait for it)
                     uint32_t v[4][32];
 #pragma unroll
                     for (int q = 0; q < 4; ++q) tmem_ld_32x32(t_row + static_cast<uint32_t>(q * 32), v[q]);
@@ -930,7 +934,10 @@ __global__ void __launch_bounds__(Cfg<CG>::NUM_THREADS, 1) gemm_f32_3xtf32_kerne
                         tmem_ld_32x16(t_row + static_cast<uint32_t>(q * 16), v);
                         tmem_ld_wait();
 #pragma unroll
-                        for (int j = 0; j < 16; ++j) sum[q * 16 + j] += __uint_as_float(v[j]);
+                        for (int j = 0; j < 16; ++j) {
+                            const float x = __uint_as_float(v[j]);
+                            sum[q * 16 + j] = CG == 2 && first ? x : sum[q * 16 + j] + x;
+                        }
                     }
                 }
                 tc_fence_before_sync();
@@ -1205,12 +1212,12 @@ __global__ void __launch_bounds__(Cfg<CG>::NUM_THREADS, 1) gemm_f32_3xtf32_kerne
                     // (16-byte chunk XOR row) of a 32 x 32 TMA box, and one lane issues a bulk
                     // tensor store.  The copy engine writes whole lines and clips the box at the
                     // edges of C; the warp's LSU work is eight 16-byte shared stores per chunk.
-                    // The unit's last tile has the rings to itself (its MMAs are done, no load
-                    // follows): all four boxes are staged side by side and leave together.
-                    // Otherwise a warp's boxes go through its own buffer (two of them in the one-CTA
+                    // In the one-CTA form the unit's last tile has the rings to itself (its MMAs are
+                    // done, no load follows): all four boxes are staged side by side and leave
+                    // together.  Otherwise a warp's boxes go through its own buffer (two of them in the one-CTA
                     // form, which has half the epilogue warps), each after the one before it in that
                     // buffer has been read.
-                    const bool last = seg == n_seg - 1;
+                    const bool last = CG == 1 && seg == n_seg - 1;
                     constexpr int OWN = CG == 1 ? 2 : 1;
                     uint8_t *base = last ? tiles + epi_warp * (4 * OUT_STAGING_WARP_BYTES)
                                          : tiles + OUT_STAGING_OFFSET + epi_warp * (OWN * OUT_STAGING_WARP_BYTES);
@@ -1277,7 +1284,7 @@ __global__ void __launch_bounds__(Cfg<CG>::NUM_THREADS, 1) gemm_f32_3xtf32_kerne
                         }
                         __syncwarp();
                     }
-                } else if (args.c_sj == 1) {
+                } else if (RAGGED && args.c_sj == 1) {
                     // Rows of C that start anywhere: the same staging, stored 32 adjacent words at a
                     // time (a thread storing its own row makes every instruction touch 32 lines).
                     uint8_t *stg = tiles + OUT_STAGING_OFFSET + epi_warp * OUT_STAGING_WARP_BYTES;
@@ -1595,16 +1602,20 @@ int launch_cg(const Problem &p, TcArgs &args, int sms, int streamk_opt, int piec
     args.total_tiles = args.tiles_m * args.tiles_n * args.B;
     // Per-device launch set-up, done once; several host threads may arrive here together.
     static std::mutex setup_mu;
-    static bool attr_set[2][64] = {{false}};
+    static bool attr_set[3][64] = {{false}};
     static int max_clusters[64] = {0};
     const int prof = (args.prof != nullptr && profile_level() == 1) ? 1 : 0;
-    auto kernel = prof ? gemm_f32_3xtf32_kernel<CG, true> : gemm_f32_3xtf32_kernel<CG, false>;
+    const bool ragged = !args.c_tma && args.c_sj == 1;
+    auto kernel = prof     ? gemm_f32_3xtf32_kernel<CG, true, false>
+                  : ragged ? gemm_f32_3xtf32_kernel<CG, false, true>
+                           : gemm_f32_3xtf32_kernel<CG, false, false>;
+    const int which = prof ? 1 : ragged ? 2 : 0;
     {
         std::lock_guard<std::mutex> lk(setup_mu);
-        if (!attr_set[prof][p.device & 63]) {
+        if (!attr_set[which][p.device & 63]) {
             cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
             if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute(smem)");
-            attr_set[prof][p.device & 63] = true;
+            attr_set[which][p.device & 63] = true;
         }
     }
     cudaLaunchConfig_t cfg{};
