@@ -39,6 +39,41 @@ struct Epilogue {
 };
 inline Epilogue epilogue_of(const Problem &p) { return Epilogue{p.d, p.d_sb, p.d_si, p.d_sj, p.act}; }
 
+// A kernel launched by launch_after() may be set up on the GPU before the one in front of it on the
+// stream has ended.  Every thread of every kernel of this library waits here, before it touches
+// memory, until that kernel is complete and its writes can be seen; a kernel launched in the
+// ordinary way passes through.  Worth 1.5 to 2 us a kernel: the six products of an attention block
+// 98 -> 85 us, a small conv layer forward and backward 76 -> 56, LSTM gates 14.3 -> 10.6.  (No kernel
+// calls the next one in early with griddepcontrol.launch_dependents: blocks that wait next to working
+// ones cost more than they gain, 512^3 15.0 us instead of 12.0, the conv layer 62.)
+__device__ __forceinline__ void after_previous_kernel() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+struct Launch {
+    dim3 grid, block;
+    size_t smem;
+    cudaStream_t stream;
+    dim3 cluster = dim3(1, 1, 1);
+};
+// Launches with programmatic dependence on the stream's previous kernel.
+template <typename... Params, typename... Args>
+cudaError_t launch_after(void (*kernel)(Params...), const Launch &l, const Args &...args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = l.grid;
+    cfg.blockDim = l.block;
+    cfg.dynamicSmemBytes = l.smem;
+    cfg.stream = l.stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = l.cluster.x;
+    attr[1].val.clusterDim.y = l.cluster.y;
+    attr[1].val.clusterDim.z = l.cluster.z;
+    cfg.attrs = attr;
+    cfg.numAttrs = l.cluster.x * l.cluster.y * l.cluster.z > 1 ? 2 : 1;
+    return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
 // Error word written by kernels whose bounded waits gave up.  One per device,
 // in ordinary global memory owned by the library.
 struct DeviceStatus {

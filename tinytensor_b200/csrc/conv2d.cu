@@ -63,6 +63,7 @@ struct alignas(sizeof(U) * 4 <= 16 ? sizeof(U) * 4 : 16) Vec4 {
 template <typename U>
 __global__ void __launch_bounds__(256) im2col_kernel(const U *__restrict__ x, U *__restrict__ cols, ConvGeom g,
                                                      long long b0) {
+    after_previous_kernel();
     const long long hw0 = (static_cast<long long>(blockIdx.x) * 256 + threadIdx.x) * 4;
     if (hw0 >= g.hw) return;
     int hs[4], ws[4];
@@ -99,6 +100,7 @@ __global__ void __launch_bounds__(256) im2col_kernel(const U *__restrict__ x, U 
 template <typename T, bool UNIT, int KT>
 __global__ void __launch_bounds__(256) col2im_kernel(const T *__restrict__ cols, T *__restrict__ gx, ConvGeom g,
                                                      long long b0) {
+    after_previous_kernel();
     using A = typename SumOf<T>::type;
     const int pix = blockIdx.x * 256 + threadIdx.x;  // grid: (pixel blocks, C_in, batch items of this group)
     if (pix >= g.H_in * g.W_in) return;
@@ -162,6 +164,7 @@ __global__ void __launch_bounds__(256) col2im_kernel(const T *__restrict__ cols,
 template <typename T>
 __global__ void __launch_bounds__(256) sum_parts_kernel(const T *__restrict__ part, T *__restrict__ out, long long n,
                                                         int parts, int accumulate) {
+    after_previous_kernel();
     using A = typename SumOf<T>::type;
     const long long i = static_cast<long long>(blockIdx.x) * 256 + threadIdx.x;
     if (i >= n) return;
@@ -176,6 +179,7 @@ __global__ void __launch_bounds__(256) sum_parts_kernel(const T *__restrict__ pa
 template <typename T>
 __global__ void __launch_bounds__(256) channel_sum_kernel(const T *__restrict__ go, T *__restrict__ part,
                                                           long long C_out, long long hw) {
+    after_previous_kernel();
     using A = std::conditional_t<std::is_floating_point_v<T>, double, typename SumOf<T>::type>;
     __shared__ A red[256];
     const long long m = blockIdx.x, b = blockIdx.y;
@@ -195,6 +199,7 @@ __global__ void __launch_bounds__(256) channel_sum_kernel(const T *__restrict__ 
 template <typename U>
 __global__ void __launch_bounds__(256) pad_rows_kernel(const U *__restrict__ src, U *__restrict__ dst, long long rows,
                                                        long long cols, long long pitch) {
+    after_previous_kernel();
     const long long i = static_cast<long long>(blockIdx.x) * 256 + threadIdx.x;
     if (i >= rows * pitch) return;
     const long long r = i / pitch, c = i % pitch;
@@ -204,8 +209,7 @@ __global__ void __launch_bounds__(256) pad_rows_kernel(const U *__restrict__ src
 template <typename U>
 int launch_im2col(const void *x, void *cols, const ConvGeom &g, long long b0, long long nb, cudaStream_t st) {
     dim3 grid(static_cast<unsigned>((g.hw + 1023) / 1024), static_cast<unsigned>(g.C_in), static_cast<unsigned>(nb));
-    im2col_kernel<U><<<grid, 256, 0, st>>>(static_cast<const U *>(x), static_cast<U *>(cols), g, b0);
-    cudaError_t e = cudaGetLastError();
+    cudaError_t e = launch_after(im2col_kernel<U>, {grid, 256, 0, st}, static_cast<const U *>(x), static_cast<U *>(cols), g, b0);
     note_launch(-1, 1);
     return e == cudaSuccess ? TTB_OK : cuda_fail(e, "im2col_kernel launch");
 }
@@ -225,32 +229,21 @@ int typed_col2im(const void *cols, void *gx, const ConvGeom &g, long long b0, lo
               static_cast<unsigned>(g.C_in), static_cast<unsigned>(nb));
     const T *src = static_cast<const T *>(cols);
     T *dst = static_cast<T *>(gx);
-    if (g.S == 1) {
-        if (g.K == 3)
-            col2im_kernel<T, true, 3><<<grid, 256, 0, st>>>(src, dst, g, b0);
-        else if (g.K == 5)
-            col2im_kernel<T, true, 5><<<grid, 256, 0, st>>>(src, dst, g, b0);
-        else
-            col2im_kernel<T, true, 0><<<grid, 256, 0, st>>>(src, dst, g, b0);
-    } else {
-        if (g.K == 3)
-            col2im_kernel<T, false, 3><<<grid, 256, 0, st>>>(src, dst, g, b0);
-        else if (g.K == 5)
-            col2im_kernel<T, false, 5><<<grid, 256, 0, st>>>(src, dst, g, b0);
-        else
-            col2im_kernel<T, false, 0><<<grid, 256, 0, st>>>(src, dst, g, b0);
-    }
-    cudaError_t e = cudaGetLastError();
+    auto kernel = g.S == 1 ? (g.K == 3   ? col2im_kernel<T, true, 3>
+                              : g.K == 5 ? col2im_kernel<T, true, 5>
+                                         : col2im_kernel<T, true, 0>)
+                           : (g.K == 3   ? col2im_kernel<T, false, 3>
+                              : g.K == 5 ? col2im_kernel<T, false, 5>
+                                         : col2im_kernel<T, false, 0>);
+    cudaError_t e = launch_after(kernel, {grid, 256, 0, st}, src, dst, g, b0);
     note_launch(-1, 1);
     return e == cudaSuccess ? TTB_OK : cuda_fail(e, "col2im_kernel launch");
 }
 
 template <typename T>
 int typed_sum_parts(const void *part, void *out, long long n, int parts, int accumulate, cudaStream_t st) {
-    sum_parts_kernel<T><<<static_cast<unsigned>((n + 255) / 256), 256, 0, st>>>(static_cast<const T *>(part),
-                                                                                static_cast<T *>(out), n, parts,
-                                                                                accumulate);
-    cudaError_t e = cudaGetLastError();
+    cudaError_t e = launch_after(sum_parts_kernel<T>, {static_cast<unsigned>((n + 255) / 256), 256, 0, st},
+                                 static_cast<const T *>(part), static_cast<T *>(out), n, parts, accumulate);
     note_launch(-1, 1);
     return e == cudaSuccess ? TTB_OK : cuda_fail(e, "sum_parts_kernel launch");
 }
@@ -258,8 +251,8 @@ int typed_sum_parts(const void *part, void *out, long long n, int parts, int acc
 template <typename T>
 int typed_channel_sum(const void *go, void *part, long long B, long long C_out, long long hw, cudaStream_t st) {
     dim3 grid(static_cast<unsigned>(C_out), static_cast<unsigned>(B));
-    channel_sum_kernel<T><<<grid, 256, 0, st>>>(static_cast<const T *>(go), static_cast<T *>(part), C_out, hw);
-    cudaError_t e = cudaGetLastError();
+    cudaError_t e = launch_after(channel_sum_kernel<T>, {grid, 256, 0, st}, static_cast<const T *>(go), static_cast<T *>(part),
+                                 C_out, hw);
     note_launch(-1, 1);
     return e == cudaSuccess ? TTB_OK : cuda_fail(e, "channel_sum_kernel launch");
 }
@@ -356,9 +349,9 @@ int weight_rows(const void *weight, const ConvGeom &g, int dtype, int device, cu
     int rc = workspace_slot(device, st, 3, static_cast<size_t>(g.C_out) * pitch * 4, &buf);
     if (rc != TTB_OK) return rc;
     const long long n = static_cast<long long>(g.C_out) * pitch;
-    pad_rows_kernel<uint32_t><<<static_cast<unsigned>((n + 255) / 256), 256, 0, st>>>(
-        static_cast<const uint32_t *>(weight), static_cast<uint32_t *>(buf), g.C_out, g.rows, pitch);
-    cudaError_t e = cudaGetLastError();
+    cudaError_t e = launch_after(pad_rows_kernel<uint32_t>, {static_cast<unsigned>((n + 255) / 256), 256, 0, st},
+                                 static_cast<const uint32_t *>(weight), static_cast<uint32_t *>(buf),
+                                 static_cast<long long>(g.C_out), g.rows, pitch);
     if (e != cudaSuccess) return cuda_fail(e, "pad_rows_kernel launch");
     note_launch(-1, 1);
     *w = buf;

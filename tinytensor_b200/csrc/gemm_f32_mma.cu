@@ -125,6 +125,7 @@ __global__ void __launch_bounds__(WARPS_M *WARPS_N *WARPS_K * 32, MIN_CTAS) gemm
     constexpr int PA = A_MN ? BM + 8 : BK + 4, PB = B_MN ? BN + 8 : BK + 4;
     constexpr int A_WORDS = T::A_WORDS, STAGE_WORDS = T::STAGE_WORDS;
     extern __shared__ __align__(16) float smem[];
+    after_previous_kernel();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int g = lane >> 2, t = lane & 3;
     const int wk = warp / (WARPS_M * WARPS_N);  // which half of a K block (WARPS_K == 2)
@@ -382,22 +383,10 @@ int launch_tile(const Problem &p, MmaArgs &args, int splits) {
     args.splits = splits;
     const int kb = (args.K + BK - 1) / BK;
     args.k_per_split = (kb + splits - 1) / splits * BK;
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(static_cast<unsigned>((p.M + BN - 1) / BN), static_cast<unsigned>((p.N + BM - 1) / BM),
-                       static_cast<unsigned>(p.B * splits));
-    cfg.blockDim = dim3(T::THREADS);
-    cfg.dynamicSmemBytes = bytes;
-    cfg.stream = p.stream;
-    cudaLaunchAttribute attr[1];
-    if (splits > 1) {
-        attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = 1;
-        attr[0].val.clusterDim.y = 1;
-        attr[0].val.clusterDim.z = static_cast<unsigned>(splits);
-        cfg.attrs = attr;
-        cfg.numAttrs = 1;
-    }
-    cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, args);
+    const dim3 grid(static_cast<unsigned>((p.M + BN - 1) / BN), static_cast<unsigned>((p.N + BM - 1) / BM),
+                    static_cast<unsigned>(p.B * splits));
+    const cudaError_t e =
+        launch_after(kernel, {grid, T::THREADS, bytes, p.stream, dim3(1, 1, static_cast<unsigned>(splits))}, args);
     return e == cudaSuccess ? TTB_OK : cuda_fail(e, "gemm_f32_mma_kernel launch");
 }
 

@@ -506,6 +506,7 @@ __global__ void __launch_bounds__(Cfg<CG>::NUM_THREADS, 1) gemm_f32_3xtf32_kerne
         cluster_wait();
     }
     tc_fence_after_sync();
+    after_previous_kernel();
     const uint32_t tmem_base = tmem_base_slot;
     // A operands in tensor memory (hybrid split only): see the map at Cfg.
     const bool a_tmem = args.a_tmem != 0 && args.terms == 2 && !(args.dbg & 8);
@@ -1622,15 +1623,18 @@ int launch_cg(const Problem &p, TcArgs &args, int sms, int streamk_opt, int piec
     cfg.blockDim = dim3(C::NUM_THREADS);
     cfg.dynamicSmemBytes = SMEM_BYTES;
     cfg.stream = p.stream;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
     int units = sms / CG;  // CTAs (CG = 1) or CTA pairs (CG = 2) resident at once
     if (CG == 2) {
-        attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = 2;
-        attr[0].val.clusterDim.y = 1;
-        attr[0].val.clusterDim.z = 1;
-        cfg.attrs = attr;
-        cfg.numAttrs = 1;
+        attr[1].id = cudaLaunchAttributeClusterDimension;
+        attr[1].val.clusterDim.x = 2;
+        attr[1].val.clusterDim.y = 1;
+        attr[1].val.clusterDim.z = 1;
+        cfg.numAttrs = 2;
         std::lock_guard<std::mutex> lk(setup_mu);
         if (max_clusters[p.device & 63] == 0) {
             cfg.gridDim = dim3(static_cast<unsigned>(2 * units));

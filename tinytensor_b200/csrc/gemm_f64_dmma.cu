@@ -73,6 +73,7 @@ __global__ void __launch_bounds__(THREADS, MIN_CTAS) gemm_f64_dmma_kernel(const 
     constexpr int WM = BM / 2, WN = BN / 2, MT = WM / 16, NT = WN / 8;
     constexpr int PA = T::LoadA::PITCH, PB = T::LoadB::PITCH;
     extern __shared__ __align__(16) double smem[];
+    after_previous_kernel();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int g = lane >> 2, t = lane & 3;  // MMA fragment coordinates
     const int wm = (warp >> 1) * WM, wn = (warp & 1) * WN;
@@ -222,22 +223,10 @@ int launch_tile(const Problem &p, DmmaArgs &args, int splits) {
     args.splits = splits;
     const int kb = (args.K + BK - 1) / BK;
     args.k_per_split = (kb + splits - 1) / splits * BK;
-    cudaLaunchConfig_t cfg{};
     args.col_tiles = static_cast<int>((p.M + BN - 1) / BN);
-    cfg.gridDim = dim3(static_cast<unsigned>(args.col_tiles * ((p.N + BM - 1) / BM)), static_cast<unsigned>(p.B * splits));
-    cfg.blockDim = dim3(THREADS);
-    cfg.dynamicSmemBytes = bytes;
-    cfg.stream = p.stream;
-    cudaLaunchAttribute attr[1];
-    if (splits > 1) {
-        attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = 1;
-        attr[0].val.clusterDim.y = static_cast<unsigned>(splits);
-        attr[0].val.clusterDim.z = 1;
-        cfg.attrs = attr;
-        cfg.numAttrs = 1;
-    }
-    cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, args);
+    const dim3 grid(static_cast<unsigned>(args.col_tiles * ((p.N + BM - 1) / BM)), static_cast<unsigned>(p.B * splits));
+    const cudaError_t e =
+        launch_after(kernel, {grid, THREADS, bytes, p.stream, dim3(1, static_cast<unsigned>(splits), 1)}, args);
     return e == cudaSuccess ? TTB_OK : cuda_fail(e, "gemm_f64_dmma_kernel launch");
 }
 

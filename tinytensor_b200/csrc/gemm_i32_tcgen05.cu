@@ -212,6 +212,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_i32_limb_kernel(const __g
         cluster_wait();
     }
     tc_fence_after_sync();
+    after_previous_kernel();
     const uint32_t tmem_base = tmem_base_slot;
 
     const int num_kb = (args.K + BK - 1) / BK;
@@ -648,15 +649,18 @@ int launch_i32_cg(const Problem &p, const I8Plan &pl, int dbg) {
     cfg.blockDim = dim3(NUM_THREADS);
     cfg.dynamicSmemBytes = SMEM_BYTES;
     cfg.stream = p.stream;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
     int units = sms / CG;  // CTAs, or CTA pairs, resident at once
     if (CG == 2) {
-        attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = 2;
-        attr[0].val.clusterDim.y = 1;
-        attr[0].val.clusterDim.z = 1;
-        cfg.attrs = attr;
-        cfg.numAttrs = 1;
+        attr[1].id = cudaLaunchAttributeClusterDimension;
+        attr[1].val.clusterDim.x = 2;
+        attr[1].val.clusterDim.y = 1;
+        attr[1].val.clusterDim.z = 1;
+        cfg.numAttrs = 2;
         static int max_clusters[64] = {0};
         if (max_clusters[p.device & 63] == 0) {
             cfg.gridDim = dim3(static_cast<unsigned>(2 * units));

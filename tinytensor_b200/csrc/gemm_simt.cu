@@ -104,6 +104,7 @@ __device__ __forceinline__ T finish(A acc, const Epilogue &ep, long long b, long
 
 template <typename T, int BM, int BN, int BK, int TM, int TN>
 __global__ void __launch_bounds__((BM / TM) * (BN / TN)) simt_gemm_kernel(SimtArgs p) {
+    after_previous_kernel();
     using A = typename AccOf<T>::type;
     constexpr int NT = (BM / TM) * (BN / TN);
     constexpr int TX = BN / TN;
@@ -269,6 +270,7 @@ template <typename T>
 __global__ void splitk_reduce_kernel(const T *__restrict__ part, T *__restrict__ c, long long B, long long N,
                                      long long M, int splits, long long c_sb, long long c_si, long long c_sj,
                                      Epilogue ep) {
+    after_previous_kernel();
     using A = typename AccOf<T>::type;
     const long long total = B * N * M;
     for (long long idx = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; idx < total;
@@ -321,16 +323,15 @@ int launch_tile(const Problem &p, int splits, void *scratch) {
         return TTB_ELIMIT;
     }
     dim3 grid(static_cast<unsigned>(gx), static_cast<unsigned>(gy), static_cast<unsigned>(gz));
-    simt_gemm_kernel<T, BM, BN, BK, TM, TN><<<grid, (BM / TM) * (BN / TN), 0, p.stream>>>(a);
-    cudaError_t e = cudaGetLastError();
+    cudaError_t e = launch_after(simt_gemm_kernel<T, BM, BN, BK, TM, TN>, {grid, (BM / TM) * (BN / TN), 0, p.stream}, a);
     if (e != cudaSuccess) return cuda_fail(e, "simt_gemm_kernel launch");
     if (splits > 1) {
         const long long total = p.B * p.N * p.M;
         const int blocks = static_cast<int>((total + 255) / 256 < 4096 ? (total + 255) / 256 : 4096);
-        splitk_reduce_kernel<T><<<blocks, 256, 0, p.stream>>>(static_cast<const T *>(scratch),
-                                                              static_cast<T *>(p.c), p.B, p.N, p.M, splits,
-                                                              p.c_sb, p.c_si, p.c_sj, epilogue_of(p));
-        e = cudaGetLastError();
+        e = launch_after(splitk_reduce_kernel<T>, {static_cast<unsigned>(blocks), 256, 0, p.stream},
+                         static_cast<const T *>(scratch), static_cast<T *>(p.c), static_cast<long long>(p.B),
+                         static_cast<long long>(p.N), static_cast<long long>(p.M), splits, static_cast<long long>(p.c_sb),
+                         static_cast<long long>(p.c_si), static_cast<long long>(p.c_sj), epilogue_of(p));
         if (e != cudaSuccess) return cuda_fail(e, "splitk_reduce_kernel launch");
     }
     return TTB_OK;
@@ -359,9 +360,8 @@ int launch_outer(const Problem &p, const SimtArgs &a, int sms, bool vec) {
     if (row_blocks > 0x7FFFFFFFLL || col_blocks > 65535) return 1;
     auto kernel = tall ? (vec ? skinny::outer_kernel<T, KT, 64, true> : skinny::outer_kernel<T, KT, 64, false>)
                        : (vec ? skinny::outer_kernel<T, KT, 16, true> : skinny::outer_kernel<T, KT, 16, false>);
-    kernel<<<dim3(static_cast<unsigned>(row_blocks), static_cast<unsigned>(col_blocks), static_cast<unsigned>(p.B)), 256, 0,
-             p.stream>>>(a);
-    cudaError_t e = cudaGetLastError();
+    const dim3 grid(static_cast<unsigned>(row_blocks), static_cast<unsigned>(col_blocks), static_cast<unsigned>(p.B));
+    cudaError_t e = launch_after(kernel, {grid, 256, 0, p.stream}, a);
     if (e != cudaSuccess) return cuda_fail(e, "outer_kernel launch");
     note_launch(TTB_VARIANT_SIMT_SKINNY, 1);
     return TTB_OK;
@@ -379,8 +379,7 @@ int launch_row_dot(const Problem &p, const SimtArgs &a, int m, int sms) {
     long long groups = (p.N + 31) / 32;
     const long long cap = (2LL * sms + p.B - 1) / p.B;  // about two CTAs of 32 warps per SM
     if (groups > cap) groups = cap;
-    kernel<<<dim3(static_cast<unsigned>(groups), static_cast<unsigned>(p.B)), 1024, bs_bytes, p.stream>>>(a, m);
-    e = cudaGetLastError();
+    e = launch_after(kernel, {dim3(static_cast<unsigned>(groups), static_cast<unsigned>(p.B)), 1024, bs_bytes, p.stream}, a, m);
     if (e != cudaSuccess) return cuda_fail(e, "row_dot_kernel launch");
     note_launch(TTB_VARIANT_SIMT_SKINNY, 1);
     return TTB_OK;
@@ -400,20 +399,8 @@ int launch_col_stream(const Problem &p, SimtArgs a, int m, int sms, bool vec) {
     a.k_per_split = (p.K + splits - 1) / splits;
     auto kernel = lx == 8 ? (vec ? skinny::col_stream_kernel<T, MC, 8, true> : skinny::col_stream_kernel<T, MC, 8, false>)
                           : (vec ? skinny::col_stream_kernel<T, MC, 32, true> : skinny::col_stream_kernel<T, MC, 32, false>);
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(static_cast<unsigned>(row_blocks), static_cast<unsigned>(splits), static_cast<unsigned>(p.B));
-    cfg.blockDim = dim3(256);
-    cfg.stream = p.stream;
-    cudaLaunchAttribute attr[1];
-    if (splits > 1) {
-        attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = 1;
-        attr[0].val.clusterDim.y = static_cast<unsigned>(splits);
-        attr[0].val.clusterDim.z = 1;
-        cfg.attrs = attr;
-        cfg.numAttrs = 1;
-    }
-    cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, a, m);
+    const dim3 grid(static_cast<unsigned>(row_blocks), static_cast<unsigned>(splits), static_cast<unsigned>(p.B));
+    cudaError_t e = launch_after(kernel, {grid, 256, 0, p.stream, dim3(1, static_cast<unsigned>(splits), 1)}, a, m);
     if (e != cudaSuccess) return cuda_fail(e, "col_stream_kernel launch");
     note_launch(TTB_VARIANT_SIMT_SKINNY, 1);
     return TTB_OK;

@@ -65,6 +65,7 @@ __device__ __forceinline__ void stage(Get get, Put put) {
 // shared memory m_cols x K accumulator words (the rhs transposed, staged once per CTA).
 template <typename T, int MC>
 __global__ void __launch_bounds__(1024) row_dot_kernel(SimtArgs p, int m_cols) {
+    after_previous_kernel();
     using A = typename AccOf<T>::type;
     extern __shared__ __align__(16) unsigned char skinny_smem[];
     A *bs = reinterpret_cast<A *>(skinny_smem);  // [j][k]
@@ -124,6 +125,7 @@ __global__ void __launch_bounds__(1024) row_dot_kernel(SimtArgs p, int m_cols) {
 // kernel for the reduction) -> 12.6 us = 5.3 TB/s.
 template <typename T, int MC, int LX, bool VEC>
 __global__ void __launch_bounds__(256) col_stream_kernel(SimtArgs p, int m_cols) {
+    after_previous_kernel();
     using A = typename AccOf<T>::type;
     constexpr int RY = 256 / LX;                                  // threads along K
     constexpr int COLS = LX * 4;                                  // rows i of this CTA
@@ -246,6 +248,7 @@ __global__ void __launch_bounds__(256) col_stream_kernel(SimtArgs p, int m_cols)
 // VEC: rows of C start on a four-element boundary.  grid (row blocks, column blocks, B).
 template <typename T, int KT, int ROWS, bool VEC>
 __global__ void __launch_bounds__(256) outer_kernel(SimtArgs p) {
+    after_previous_kernel();
     using A = typename AccOf<T>::type;
     __shared__ __align__(16) A as[ROWS][KT];
     __shared__ __align__(16) A bs[KT][256 + 16 / sizeof(A)];

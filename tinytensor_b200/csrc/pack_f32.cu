@@ -25,6 +25,7 @@ struct PackOne {
 };
 
 __global__ void __launch_bounds__(256) pack_rows_kernel(PackOne a, PackOne b) {
+    after_previous_kernel();
     const int lane = threadIdx.x & 31;
     const long long warp0 = static_cast<long long>(blockIdx.x) * 8 + (threadIdx.x >> 5);
     for (long long w = warp0; w < a.total_rows + b.total_rows; w += static_cast<long long>(gridDim.x) * 8) {
@@ -95,8 +96,7 @@ int pack_f32_operands(Problem *p) {
     sm_count(p->device, &sms);
     long long blocks = (rows + 7) / 8;
     if (blocks > 8LL * sms) blocks = 8LL * sms;
-    pack_rows_kernel<<<static_cast<unsigned>(blocks), 256, 0, p->stream>>>(pa, pb);
-    cudaError_t e = cudaGetLastError();
+    cudaError_t e = launch_after(pack_rows_kernel, {static_cast<unsigned>(blocks), 256, 0, p->stream}, pa, pb);
     if (e != cudaSuccess) return cuda_fail(e, "pack_rows_kernel launch");
     note_launch(-1, 1);
     if (da != nullptr) {
