@@ -79,7 +79,7 @@ enum ttb_variant {
     TTB_VARIANT_TCGEN05_2CTA = 5, /* f32: tcgen05 cta_group::2 (CTA pairs) */
     TTB_VARIANT_TCGEN05_I8LIMB = 6, /* i32: exact mod 2^32 from ten u8 x u8 tcgen05 products of byte planes */
     TTB_VARIANT_SIMT_SKINNY = 7,  /* one dim <= 16: streaming kernels (reported only; not forceable) */
-    TTB_VARIANT_MMA_F32 = 8       /* f32: mma.sync, same split precision, small tiles, any view */
+    TTB_VARIANT_MMA_F32 = 8       /* f32: mma.sync, three bf16 parts a word, small tiles, any view */
 };
 
 /* ---- the hot path -------------------------------------------------------
