@@ -142,3 +142,26 @@ def test_bad_arguments_raise(ttb):
         ttb.conv2d(x, torch.ones(4, 3, 3, 3, device="cuda"), None, 0, 0)  # stride 0
     with pytest.raises(ttb.TTBError):
         ttb.conv2d(x, torch.ones(4, 3, 3, 3, device="cuda", dtype=torch.float64))
+
+
+@pytest.mark.parametrize("dt", [np.float32, np.float64, np.int32, np.uint8])
+@pytest.mark.parametrize("geom", [
+    dict(B=37, C_in=6, C_out=5, H=7, W=9, K=1, S=1, P=0),       # rows that TMA cannot describe, parts beyond two groups of 16
+    dict(B=16, C_in=72, C_out=96, H=12, W=14, K=1, S=1, P=0),   # the input as columns
+    dict(B=16, C_in=72, C_out=96, H=13, W=13, K=1, S=1, P=0),   # copied: the products are large and the rows unaligned
+    dict(B=3, C_in=4, C_out=8, H=9, W=9, K=1, S=2, P=0),
+    dict(B=2, C_in=4, C_out=8, H=9, W=9, K=1, S=1, P=1),
+    dict(B=5, C_in=3, C_out=70, H=32, W=32, K=5, S=1, P=2),     # weight rows of 75: small enough to stay unpadded, and
+    dict(B=5, C_in=7, C_out=128, H=64, W=64, K=3, S=1, P=1),    # of 63: padded
+])
+def test_columns_in_place_and_unpadded_weights(ttb, oracle, dt, geom):
+    rng = np.random.default_rng(66)
+    g = geom
+    x, w = _draw(rng, dt, (g["B"], g["C_in"], g["H"], g["W"])), _draw(rng, dt, (g["C_out"], g["C_in"], g["K"], g["K"]))
+    b = _draw(rng, dt, (g["C_out"],))
+    y = host(ttb.conv2d(dev(x), dev(w), dev(b), g["S"], g["P"]))
+    _close(y, oracle.conv2d_forward(x, w, b, g["S"], g["P"]), dt)
+    go = _draw(rng, dt, y.shape)
+    got = ttb.conv2d_backward(dev(go), dev(x), dev(w), g["S"], g["P"])
+    for have, want in zip(got, oracle.conv2d_backward(go, x, w, g["S"], g["P"])):
+        _close(host(have), want, dt)

@@ -14,6 +14,8 @@
 //                           col2im in gather form: one thread per input pixel adds its <= K*K
 //                           contributions in (p, q) order, the order the reference's CPU loop
 //                           adds them in, without atomics or races.
+// A 1 x 1 kernel of stride 1 without padding needs no columns: they are the input itself, and grad_x's
+// are grad_x.
 // All kernels here are HBM-bound copies / short sums; their algorithmic bytes are the tensors
 // they read and write once.
 #include <cuda_runtime.h>
@@ -160,17 +162,38 @@ __global__ void __launch_bounds__(256) col2im_kernel(const T *__restrict__ cols,
     gx[(((b0 + bz) * g.C_in + c) * g.H_in + hi) * static_cast<long long>(g.W_in) + wi] = static_cast<T>(s);
 }
 
-// out[i] = (accumulate ? out[i] : 0) + part[0][i] + part[1][i] + ... in that order.
+// out[i] = (accumulate ? out[i] : 0) + part[0][i] + part[1][i] + ... in that order, for the `n` elements
+// of one array and then those of another.  Sixteen parts are loaded before the first is added: the
+// sum is a chain, its loads need not be one.
 template <typename T>
-__global__ void __launch_bounds__(256) sum_parts_kernel(const T *__restrict__ part, T *__restrict__ out, long long n,
-                                                        int parts, int accumulate) {
+struct SumArray {
+    const T *part;
+    T *out;
+    long long n;
+    int parts, accumulate;
+};
+template <typename T>
+__global__ void __launch_bounds__(256) sum_parts_kernel(SumArray<T> x, SumArray<T> y) {
     after_previous_kernel();
     using A = typename SumOf<T>::type;
-    const long long i = static_cast<long long>(blockIdx.x) * 256 + threadIdx.x;
-    if (i >= n) return;
-    A s = accumulate ? static_cast<A>(out[i]) : A(0);
-    for (int b = 0; b < parts; ++b) s = s + static_cast<A>(part[b * n + i]);
-    out[i] = static_cast<T>(s);
+    long long i = static_cast<long long>(blockIdx.x) * 256 + threadIdx.x;
+    if (i >= x.n) {
+        i -= x.n;
+        x = y;
+        if (i >= x.n) return;
+    }
+    A s = x.accumulate ? static_cast<A>(x.out[i]) : A(0);
+    const T *src = x.part + i;
+    int b = 0;
+    for (; b + 16 <= x.parts; b += 16) {
+        T v[16];
+#pragma unroll
+        for (int u = 0; u < 16; ++u) v[u] = src[(b + u) * x.n];
+#pragma unroll
+        for (int u = 0; u < 16; ++u) s = s + static_cast<A>(v[u]);
+    }
+    for (; b < x.parts; ++b) s = s + static_cast<A>(src[b * x.n]);
+    x.out[i] = static_cast<T>(s);
 }
 
 // part[b][m] = sum over h, w of g_out[b][m][h][w]: one CTA per (channel, batch item); the batch
@@ -241,9 +264,11 @@ int typed_col2im(const void *cols, void *gx, const ConvGeom &g, long long b0, lo
 }
 
 template <typename T>
-int typed_sum_parts(const void *part, void *out, long long n, int parts, int accumulate, cudaStream_t st) {
-    cudaError_t e = launch_after(sum_parts_kernel<T>, {static_cast<unsigned>((n + 255) / 256), 256, 0, st},
-                                 static_cast<const T *>(part), static_cast<T *>(out), n, parts, accumulate);
+int typed_sum_parts(const void *part, void *out, long long n, int parts, int accumulate, cudaStream_t st,
+                    const void *part2, void *out2, long long n2, int parts2) {
+    const SumArray<T> x{static_cast<const T *>(part), static_cast<T *>(out), n, parts, accumulate};
+    const SumArray<T> y{static_cast<const T *>(part2), static_cast<T *>(out2), n2, parts2, 0};
+    cudaError_t e = launch_after(sum_parts_kernel<T>, {static_cast<unsigned>((n + n2 + 255) / 256), 256, 0, st}, x, y);
     note_launch(-1, 1);
     return e == cudaSuccess ? TTB_OK : cuda_fail(e, "sum_parts_kernel launch");
 }
@@ -325,6 +350,17 @@ long long chunk_batches(const ConvGeom &g, long long B, size_t es) {
     return nb < B ? nb : B;
 }
 
+// The columns of a 1 x 1 kernel of stride 1 without padding are the input, image for image.  They are
+// used in place unless a product large enough for TMA's kernels would meet rows that are not a
+// multiple of 16 bytes: then the copy into padded rows is the smaller cost.
+bool columns_are_input(const ConvGeom &g, long long nb, int dtype, size_t es, const void *images, const void *grads) {
+    if (g.K != 1 || g.S != 1 || g.P != 0) return false;
+    if (dtype != TTB_F32 && dtype != TTB_I32) return true;
+    const bool aligned = static_cast<size_t>(g.hw) * es % 16 == 0 && reinterpret_cast<uintptr_t>(images) % 16 == 0 &&
+                         reinterpret_cast<uintptr_t>(grads) % 16 == 0;
+    return aligned || static_cast<double>(nb) * g.C_out * g.C_in * g.hw < 16777216.0;
+}
+
 int select_device(int device) {
     int ndev = 0;
     cudaError_t e = cudaGetDeviceCount(&ndev);
@@ -337,13 +373,18 @@ int select_device(int device) {
     return e == cudaSuccess ? TTB_OK : cuda_fail(e, "cudaSetDevice");
 }
 
-// Weight rows for the tensor-core path: TMA needs a 16-byte row pitch, so an f32 weight
-// matrix whose row length C_in*K*K is not a multiple of 4 is copied once into padded rows.
-int weight_rows(const void *weight, const ConvGeom &g, int dtype, int device, cudaStream_t st, const void **w,
+// Weight rows for the tcgen05 kernel: TMA needs a 16-byte row pitch, so an f32 weight matrix whose
+// row length C_in*K*K is not a multiple of 4 is copied once into padded rows.  Products of less than 2^25
+// multiply-adds, or 2^29 with few output channels, are faster on the mma.sync kernel, which takes any
+// pitch, than the copy and the tcgen05 kernel together (2^24.8, 96 channels, 16.1 -> 13.8 us forward;
+// 2^26.6, 100 channels, 19.4 against 22.2 the other way).
+int weight_rows(const void *weight, const ConvGeom &g, long long nb, int dtype, int device, cudaStream_t st, const void **w,
                 long long *w_pitch) {
     *w = weight;
     *w_pitch = g.rows;
     if (dtype != TTB_F32 || (g.rows & 3) == 0) return TTB_OK;
+    const double work = static_cast<double>(nb) * g.C_out * static_cast<double>(g.rows) * static_cast<double>(g.hw);
+    if (work < (g.C_out < 64 ? 536870912.0 : 33554432.0)) return TTB_OK;
     const long long pitch = (g.rows + 3) / 4 * 4;
     void *buf = nullptr;
     int rc = workspace_slot(device, st, 3, static_cast<size_t>(g.C_out) * pitch * 4, &buf);
@@ -379,25 +420,31 @@ extern "C" TTB_API int ttb_conv2d_forward(const void *input, const void *weight,
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const long long B = desc->batch;
     const long long nb_max = chunk_batches(g, B, es);
+    const bool in_place = columns_are_input(g, nb_max, dtype, es, input, out);
     void *cols = nullptr;
-    rc = workspace_slot(device_id, st, 1, static_cast<size_t>(nb_max) * g.rows * g.pitch * es, &cols);
-    if (rc != TTB_OK) return rc;
+    if (!in_place) {
+        rc = workspace_slot(device_id, st, 1, static_cast<size_t>(nb_max) * g.rows * g.pitch * es, &cols);
+        if (rc != TTB_OK) return rc;
+    }
+    const long long pitch = in_place ? g.hw : g.pitch;
     const void *w = nullptr;
     long long w_pitch = 0;
-    rc = weight_rows(weight, g, dtype, device_id, st, &w, &w_pitch);
+    rc = weight_rows(weight, g, nb_max, dtype, device_id, st, &w, &w_pitch);
     if (rc != TTB_OK) return rc;
     for (long long b0 = 0; b0 < B; b0 += nb_max) {
         const long long nb = b0 + nb_max <= B ? nb_max : B - b0;
-        rc = im2col(input, cols, g, b0, nb, es, st);
-        if (rc != TTB_OK) return rc;
+        if (!in_place) {
+            rc = im2col(input, cols, g, b0, nb, es, st);
+            if (rc != TTB_OK) return rc;
+        }
         Problem p{};
         p.a = w;  // the same weight matrix for every batch item: batch stride 0
         p.a_sb = 0;
         p.a_si = w_pitch;
         p.a_sk = 1;
-        p.b = cols;
-        p.b_sb = g.rows * g.pitch;
-        p.b_sk = g.pitch;
+        p.b = in_place ? static_cast<const char *>(input) + static_cast<size_t>(b0) * g.C_in * g.hw * es : cols;
+        p.b_sb = g.rows * pitch;
+        p.b_sk = pitch;
         p.b_sj = 1;
         p.c = static_cast<char *>(out) + static_cast<size_t>(b0) * g.C_out * g.hw * es;
         p.c_sb = g.C_out * g.hw;
@@ -438,24 +485,38 @@ extern "C" TTB_API int ttb_conv2d_backward(const void *grad_out, const void *inp
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const long long B = desc->batch;
     const long long nb_max = chunk_batches(g, B, es);
+    const bool in_place = columns_are_input(g, nb_max, dtype, es, input, grad_out) &&
+                          ((dtype != TTB_F32 && dtype != TTB_I32) || reinterpret_cast<uintptr_t>(grad_input) % 16 == 0) &&
+                          grad_input != grad_out;
     void *cols = nullptr, *parts = nullptr;
-    rc = workspace_slot(device_id, st, 1, static_cast<size_t>(nb_max) * g.rows * g.pitch * es, &cols);
-    if (rc != TTB_OK) return rc;
+    if (!in_place) {
+        rc = workspace_slot(device_id, st, 1, static_cast<size_t>(nb_max) * g.rows * g.pitch * es, &cols);
+        if (rc != TTB_OK) return rc;
+    }
+    const long long pitch = in_place ? g.hw : g.pitch;
     const long long wn = static_cast<long long>(g.C_out) * g.rows;
-    // also holds the per-item channel sums of grad_bias afterwards
-    const long long parts_elems = nb_max * wn > B * g.C_out ? nb_max * wn : B * g.C_out;
+    // (with the per-item channel sums of grad_bias behind them)
+    const long long parts_elems = nb_max * wn + (grad_bias ? B * g.C_out : 0);
     rc = workspace_slot(device_id, st, 2, static_cast<size_t>(parts_elems) * es, &parts);
     if (rc != TTB_OK) return rc;
+    char *channel_parts = static_cast<char *>(parts) + static_cast<size_t>(nb_max * wn) * es;
     const void *w = nullptr;
     long long w_pitch = 0;
-    rc = weight_rows(weight, g, dtype, device_id, st, &w, &w_pitch);
+    rc = weight_rows(weight, g, nb_max, dtype, device_id, st, &w, &w_pitch);
     if (rc != TTB_OK) return rc;
+    if (grad_bias) {
+        rc = TTB_BY_DTYPE(dtype, typed_channel_sum, grad_out, channel_parts, B, static_cast<long long>(g.C_out), g.hw, st);
+        if (rc != TTB_OK) return rc;
+    }
     for (long long b0 = 0; b0 < B; b0 += nb_max) {
         const long long nb = b0 + nb_max <= B ? nb_max : B - b0;
         const char *go = static_cast<const char *>(grad_out) + static_cast<size_t>(b0) * g.C_out * g.hw * es;
         // grad_w partials: g_out[b][C_out, HW] . columns[b]^T[HW, CKK]
-        rc = im2col(input, cols, g, b0, nb, es, st);
-        if (rc != TTB_OK) return rc;
+        const size_t first = static_cast<size_t>(b0) * g.C_in * g.H_in * g.W_in * es;
+        if (!in_place) {
+            rc = im2col(input, cols, g, b0, nb, es, st);
+            if (rc != TTB_OK) return rc;
+        }
         Problem p{};
         p.dtype = dtype;
         p.device = device_id;
@@ -465,10 +526,10 @@ extern "C" TTB_API int ttb_conv2d_backward(const void *grad_out, const void *inp
         p.a_sb = g.C_out * g.hw;
         p.a_si = g.hw;
         p.a_sk = 1;
-        p.b = cols;
-        p.b_sb = g.rows * g.pitch;
-        p.b_sk = 1;        // columns^T: k walks along a row of the columns buffer,
-        p.b_sj = g.pitch;  // j from row to row
+        p.b = in_place ? static_cast<const char *>(input) + first : cols;
+        p.b_sb = g.rows * pitch;
+        p.b_sk = 1;      // columns^T: k walks along a row of the columns buffer,
+        p.b_sj = pitch;  // j from row to row
         p.c = parts;
         p.c_sb = wn;
         p.c_si = g.rows;
@@ -478,7 +539,10 @@ extern "C" TTB_API int ttb_conv2d_backward(const void *grad_out, const void *inp
         p.M = g.rows;
         rc = dispatch_problem(p);
         if (rc != TTB_OK) return rc;
-        rc = TTB_BY_DTYPE(dtype, typed_sum_parts, parts, grad_weight, wn, static_cast<int>(nb), b0 > 0 ? 1 : 0, st);
+        // (grad_bias's sums ride along with the first group's)
+        const long long bias_n = grad_bias && b0 == 0 ? g.C_out : 0;
+        rc = TTB_BY_DTYPE(dtype, typed_sum_parts, parts, grad_weight, wn, static_cast<int>(nb), b0 > 0 ? 1 : 0, st,
+                          channel_parts, grad_bias, bias_n, static_cast<int>(B));
         if (rc != TTB_OK) return rc;
         // grad_x columns: W^T[CKK, C_out] . g_out[b][C_out, HW], overwriting the columns buffer
         Problem q{};
@@ -494,23 +558,17 @@ extern "C" TTB_API int ttb_conv2d_backward(const void *grad_out, const void *inp
         q.b_sb = g.C_out * g.hw;
         q.b_sk = g.hw;
         q.b_sj = 1;
-        q.c = cols;
-        q.c_sb = g.rows * g.pitch;
-        q.c_si = g.pitch;
+        q.c = in_place ? static_cast<char *>(grad_input) + first : cols;
+        q.c_sb = g.rows * pitch;
+        q.c_si = pitch;
         q.c_sj = 1;
         q.N = g.rows;
         q.K = g.C_out;
         q.M = g.hw;
         rc = dispatch_problem(q);
         if (rc != TTB_OK) return rc;
+        if (in_place) continue;
         rc = TTB_BY_DTYPE(dtype, typed_col2im, cols, grad_input, g, b0, nb, st);
-        if (rc != TTB_OK) return rc;
-    }
-    if (grad_bias) {
-        rc = TTB_BY_DTYPE(dtype, typed_channel_sum, grad_out, parts, B, static_cast<long long>(g.C_out), g.hw, st);
-        if (rc != TTB_OK) return rc;
-        rc = TTB_BY_DTYPE(dtype, typed_sum_parts, parts, grad_bias, static_cast<long long>(g.C_out), static_cast<int>(B),
-                          0, st);
         if (rc != TTB_OK) return rc;
     }
     return TTB_OK;
